@@ -14,6 +14,7 @@
 #include "../../include/dd_gpu.h"
 #include "dd_common.cuh"
 #include "kernels.cuh"
+#include "prune_core.cuh"
 #include "search_core.cuh"
 #include "semisort.cuh"
 #include "sort_emul.cuh"
@@ -38,7 +39,10 @@ struct dd_index {
   uint32_t* new_out = nullptr;
   float* new_key = nullptr;  // distances of new_out's entries (fast form)
   float* row_key = nullptr;  // n x Rp: each graph entry's distance to its row's point (fast form)
+  uint32_t* row_meta = nullptr;  // n: each row's degree and pruned prefix (fast form)
+  int* norms = nullptr;          // n: |x|^2 of the rows (fast form, integer data)
   bool row_key_ok = false;
+  ReverseFork fork;              // hub targets' stream beside the other reverse edges
   uint32_t* stat_vis = nullptr;
   uint32_t* stat_cmps = nullptr;
   uint32_t* sort_t[2] = {nullptr, nullptr};  // semisort ping-pong buffers
@@ -229,7 +233,7 @@ std::vector<std::pair<uint64_t, uint64_t>> schedule(uint64_t n, uint64_t max_bui
 
 int ensure_build_scratch(dd_index* h, uint64_t B) {
   if (!h->counters) {
-    CK(dalloc(&h->counters, 8));
+    CK(dalloc(&h->counters, kCounters));
     CK(dalloc(&h->block_sums, kScanBlocks + 1));
     CK(dalloc(&h->acc, 8));
   }
@@ -329,6 +333,8 @@ ReverseScratch make_rs(dd_index* h, int res) {
   rs.heads = h->heads;
   rs.counters = h->counters;
   rs.big = h->big;
+  rs.list = h->flags;  // free once the segment heads are listed
+  rs.list_cap = h->bcap * h->Rp;
   rs.gcand = h->gcand;
   rs.gkey = h->gkey;
   rs.gpos = h->gpos;
@@ -529,7 +535,10 @@ int pass_rounds(dd_index* h, const std::vector<std::pair<uint64_t, uint64_t>>& r
                 TuneResult* tune) {
   IndexView ix = view(h);
   if (bp.screen) attach_screen(h, &ix);
-  if (bp.fast) ix.fgroup_lg = fast_fgroup(h);
+  if (bp.fast) {
+    ix.fgroup_lg = fast_fgroup(h);
+    ix.norms = h->norms;
+  }
   for (size_t r = 0; r < rounds.size(); r++) {
     const auto& rd = rounds[r];
     uint64_t B = rd.second > rd.first ? rd.second - rd.first : 0;
@@ -543,6 +552,7 @@ int pass_rounds(dd_index* h, const std::vector<std::pair<uint64_t, uint64_t>>& r
     ra.new_out = h->new_out;
     ra.new_key = bp.fast ? h->new_key : nullptr;
     ra.row_key = bp.fast ? h->row_key : nullptr;
+    ra.row_meta = bp.fast ? h->row_meta : nullptr;
     ra.stat_vis = h->stat_vis;
     ra.stat_cmps = h->stat_cmps;
     ra.vis_all = h->vis_all;
@@ -556,7 +566,7 @@ int pass_rounds(dd_index* h, const std::vector<std::pair<uint64_t, uint64_t>>& r
     }
     if (bp.fast && bp.squeue) ra.qsearch = h->queues + qbase + 2 * r;
     if (bp.fast && bp.pqueue) ra.qprune = h->queues + qbase + 2 * r + 1;
-    CK(cudaMemsetAsync(h->counters, 0, 8 * 4, h->stream));
+    CK(cudaMemsetAsync(h->counters, 0, kCounters * 4, h->stream));
     if (pe) CK(cudaEventRecord(pe->next(), h->stream));
     launch_search(ix, ra, bp.slay, bp.splan, grid_for(bp.splan, B, h->sm_count), h->stream);
     if (pe) CK(cudaEventRecord(pe->next(), h->stream));
@@ -566,11 +576,13 @@ int pass_rounds(dd_index* h, const std::vector<std::pair<uint64_t, uint64_t>>& r
     launch_apply_rows(ix, ra, h->stream);
     SemisortScratch ss = make_ss(h);
     const int res = launch_semisort(h->new_out, B * h->Rp, h->n, ss, h->stream);
-    launch_reverse(ix, ra, make_rs(h, res), bp.fast, h->stream, h->sm_count);
-    // k_search, k_prune, k_apply_rows, k_reverse, k_reverse_big; per radix
-    // pass a histogram, three scans and a scatter; the segment heads' flags,
-    // three scans and scatter
-    h->launches += 10 + 5 * (uint64_t)((64 - __builtin_clzll(h->n > 1 ? h->n - 1 : 1) + 7) / 8);
+    ReverseScratch rs = make_rs(h, res);
+    rs.split = bp.fast && B * h->Rp >= kRevSplitPairs;
+    launch_reverse(ix, ra, rs, bp.fast, h->stream, h->sm_count, h->fork);
+    // k_search, k_prune, k_apply_rows, k_reverse, k_reverse_big, and k_rev_split,
+    // k_rev_short of split rounds; per radix pass a histogram, three scans and
+    // a scatter; the segment heads' flags, three scans and scatter
+    h->launches += 10 + (rs.split ? 2 : 0) + 5 * (uint64_t)((64 - __builtin_clzll(h->n > 1 ? h->n - 1 : 1) + 7) / 8);
     if (P->collect_stats) {
       k_accumulate<<<64, 256, 0, h->stream>>>(h->stat_vis, h->stat_cmps, (uint32_t)B, h->counters,
                                               h->acc);
@@ -599,13 +611,24 @@ int build_sequence(dd_index* h, const std::vector<std::pair<uint64_t, uint64_t>>
   CK(cudaMemsetAsync(h->graph, 0xff, h->n * h->Rp * 4ull, h->stream));
   CK(cudaMemsetAsync(h->acc, 0, 8 * 8, h->stream));
   CK(cudaMemsetAsync(h->err, 0, 4, h->stream));
-  if (bp.fast) CK(cudaMemsetAsync(h->queues, 0, h->queue_words * 4, h->stream));
+  if (bp.fast) {
+    CK(cudaMemsetAsync(h->queues, 0, h->queue_words * 4, h->stream));
+    CK(cudaMemsetAsync(h->row_meta, 0, h->n * 4ull, h->stream));
+    if (h->norms) {
+      launch_row_norms(view(h), h->norms, h->stream);
+      h->launches++;
+    }
+  }
   const uint64_t per_pass = 2 * rounds.size();
   int rc;
   if (Q->two_pass) {
     rc = pass_rounds(h, rounds, 1.0, Q, bp, 2, pe, tune);
     if (rc) return rc;
     tune = nullptr;
+    if (bp.fast) {  // rows pruned with the first pass's alpha
+      launch_clear_clean(h->row_meta, h->n, h->stream);
+      h->launches++;
+    }
   }
   rc = pass_rounds(h, rounds, Q->alpha, Q, bp, 2 + (Q->two_pass ? per_pass : 0), pe, tune);
   if (rc) return rc;
@@ -669,7 +692,7 @@ int dd_destroy(dd_index* h) {
                   h->sort_t[0], h->sort_t[1], h->sort_v[0], h->sort_v[1], h->hist, h->heads,
                   h->flags, h->counters, h->big, h->block_sums, h->acc, h->gcand, h->gkey,
                   h->gpos, h->gbits, h->granges, h->vis_all, h->ref_rows, h->row_key,
-                  h->screen, h->snorm};
+                  h->row_meta, h->norms, h->screen, h->snorm};
   for (void* p : ptrs) dfree(p);
   dfree(h->queues);
   dfree(h->qcls);
@@ -677,6 +700,10 @@ int dd_destroy(dd_index* h) {
   dfree(h->qev);
   if (h->gexec) cudaGraphExecDestroy(h->gexec);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
+  for (cudaStream_t a : h->fork.aux)
+    if (a) cudaStreamDestroy(a);
+  for (cudaEvent_t e : {h->fork.forked, h->fork.joined[0], h->fork.joined[1]})
+    if (e) cudaEventDestroy(e);
   delete h;
   return DD_OK;
 }
@@ -905,8 +932,18 @@ int build_once(dd_index* h, const dd_build_params* P, uint32_t vcap, dd_stats* s
     // the fast form keeps every graph entry's distance to its row's point
     // beside the graph, so a reverse prune needs no distance of its row
     h->scratch_gen++;
-    CK(dalloc(&h->row_key, h->n * (uint64_t)h->Rp));
+    if (!h->row_key) CK(dalloc(&h->row_key, h->n * (uint64_t)h->Rp));
+    if (!h->row_meta) CK(dalloc(&h->row_meta, h->n));
+    if (!h->norms && greedy_uses_mma(h->d, h->dtype)) CK(dalloc(&h->norms, h->n));
     h->row_key_ok = true;
+  }
+  if (bp.fast && Bmax * h->Rp >= kRevSplitPairs) {
+    if (!h->fork.forked) CK(cudaEventCreateWithFlags(&h->fork.forked, cudaEventDisableTiming));
+    for (int i = 0; i < 2; i++) {
+      if (!h->fork.aux[i]) CK(cudaStreamCreateWithFlags(&h->fork.aux[i], cudaStreamNonBlocking));
+      if (!h->fork.joined[i])
+        CK(cudaEventCreateWithFlags(&h->fork.joined[i], cudaEventDisableTiming));
+    }
   }
   rc = ensure_vis_all(h, Bmax * 2ull * vcap);
   if (rc) return rc;
@@ -1089,6 +1126,7 @@ RoundArgs shard_round_args(dd_index* h, uint64_t floor, uint64_t B, uint32_t* ro
   ra.new_out = rows;
   ra.new_key = nullptr;  // the exchanged rows carry no distances: the reverse step recomputes
   ra.row_key = nullptr;
+  ra.row_meta = nullptr;
   ra.stat_vis = h->stat_vis;
   ra.stat_cmps = h->stat_cmps;
   ra.vis_all = h->vis_all;
@@ -1176,14 +1214,14 @@ int dd_shard_apply_reverse(dd_index* h, uint64_t floor, uint64_t ceiling, const 
   const uint64_t B = ceiling - floor;
   RoundArgs ra = shard_round_args(h, floor, B, const_cast<uint32_t*>(batch_rows));
   IndexView ix = view(h);
-  CK(cudaMemsetAsync(h->counters, 0, 8 * 4, h->stream));
+  CK(cudaMemsetAsync(h->counters, 0, kCounters * 4, h->stream));
   launch_apply_rows(ix, ra, h->stream);
   SemisortScratch ss = make_ss(h);
   ss.world = (uint32_t)world;
   ss.rank = (uint32_t)rank;
   const int res = launch_semisort(batch_rows, B * h->Rp, h->n, ss, h->stream);
   ReverseScratch rs = make_rs(h, res);
-  launch_reverse(ix, ra, rs, bp.fast, h->stream, h->sm_count);
+  launch_reverse(ix, ra, rs, bp.fast, h->stream, h->sm_count, ReverseFork{});
   launch_export_rows(ix, rs.st, rs.heads, h->counters, cap, ids_out, rows_out, h->stream);
   CK(cudaGetLastError());
   uint32_t c[2] = {0, 0};

@@ -82,9 +82,11 @@ __global__ void __launch_bounds__(512) k_prune(IndexView ix, RoundArgs ra, Prune
     }
     __syncwarp();
     warp_std_sort(Pm, m);
-    warp_greedy_select_fast<DT, MT, true, TC>(ix.points, ix.stride, ix.d, p, Pm, m, ra.alpha, ix.R,
-                                    ra.new_out + b * ix.Rp, ix.Rp, Pm.sel,
-                                    ra.new_key ? ra.new_key + b * ix.Rp : nullptr);
+    const uint32_t nsel = warp_greedy_select_fast<DT, MT, true, TC>(
+        ix.points, ix.stride, ix.d, p, Pm, m, ra.alpha, ix.R, ra.new_out + b * ix.Rp, ix.Rp, Pm.sel,
+        ra.new_key ? ra.new_key + b * ix.Rp : nullptr);
+    // what the row will be once k_apply_rows has copied it
+    if (ra.row_meta && lane == 0) ra.row_meta[p] = nsel | (nsel << 16);
   }
 }
 

@@ -55,6 +55,8 @@ struct IndexView {
   // exact distance in a search step (0: one lane, the plain form; 4: chosen
   // per step from the candidate count)
   uint32_t fgroup_lg = 0;
+  // fast form builds, integer data: |x|^2 of every row (null: not computed)
+  const int* norms = nullptr;
 };
 
 // keep_vis: the query layout reserves the visited list (k_beam keeps it;
@@ -80,6 +82,9 @@ struct RoundArgs {
                          // null (the reverse step then recomputes them)
   float* row_key;        // with new_key: n x Rp, each graph entry's distance to its row's
                          // point (kept by every row write of the build), or null
+  uint32_t* row_meta;    // with row_key: n words, each row's degree (low 16 bits) and how many
+                         // of its leading entries are the selection of one prune with this
+                         // pass's alpha (high 16 bits), or null
   uint32_t* stat_vis;    // B visited-list lengths (k_search writes, k_prune reads)
   uint32_t* stat_cmps;   // B (may be null)
   uint32_t* vis_all;     // per batch point: vcap visited ids, then vcap distances
@@ -100,7 +105,14 @@ struct ReverseScratch {
   const uint32_t* heads;
   uint32_t* counters;  // [0] pairs V [1] segments T [2] pruned groups [3] prune cands
                        // [4] big segments [5] largest big candidate list
+                       // [6] / [7] segments of the short and the general prune list,
+                       // [8] / [9] their work queues
   uint32_t* big;       // segments for the CTA path
+  // segments to prune (k_rev_split): the short list from the front, the
+  // general list from the end
+  uint32_t* list;
+  uint64_t list_cap;
+  bool split = false;  // the round's targets are split by k_rev_split (kRevSplitPairs)
   // CTA path workspace, one slice per CTA (kBigSlots slices of gcap candidates):
   uint32_t* gcand;     // gcap ids
   float* gkey;         // gcap distances
@@ -115,6 +127,16 @@ constexpr int kScanBlocks = 512;
 constexpr int kGlobalStackInts = 3 * (2 * 32 + 4);
 constexpr uint32_t kRevCandCap = 256;   // per-warp shared-memory candidates (reverse)
 constexpr uint32_t kRevWarps = 2;       // warps per CTA of the reverse kernel
+constexpr uint32_t kRevShortCap = 128;  // candidates of a short reverse prune,
+constexpr uint32_t kRevShortNew = 32;   // and how many of them may be new to the row
+// Pairs of a round (batch points x row length) from which the fast form's
+// targets are split over three prunes on three streams; a smaller round's
+// targets fit the GPU's resident warps a few times over, and two kernels in
+// one stream end sooner than four in three (10k x 20 f32, rounds of 200 points
+// and 6400 pairs: 1.6 ms of reverse edges a build against 3.6 split; 100k x 64
+// f32 with every round split gains nothing below this line).
+constexpr uint64_t kRevSplitPairs = 32768;
+constexpr uint32_t kCounters = 16;      // words of ReverseScratch::counters
 constexpr uint32_t kBigThreads = 512;   // threads per CTA of the big-target path
 constexpr uint32_t kBigSlots = 148;     // CTAs (and workspace slices) of the big-target path
 
@@ -131,9 +153,19 @@ void launch_prune_round(const IndexView& ix, const RoundArgs& ra, const PruneLay
                         uint32_t vcap, const LaunchPlan& plan, int grid, bool tensor,
                         cudaStream_t st);
 void launch_apply_rows(const IndexView& ix, const RoundArgs& ra, cudaStream_t st);
-// append-or-prune per target over the segments the semisort produced
+// append-or-prune per target over the segments the semisort produced.  With
+// rs.split the hub targets and the general prunes run on streams of their
+// own beside the short ones; `st` waits for them.
+struct ReverseFork {
+  cudaStream_t aux[2] = {nullptr, nullptr};
+  cudaEvent_t forked = nullptr, joined[2] = {nullptr, nullptr};
+};
 void launch_reverse(const IndexView& ix, const RoundArgs& ra, const ReverseScratch& rs,
-                    bool tensor, cudaStream_t st, int sm_count);
+                    bool tensor, cudaStream_t st, int sm_count, const ReverseFork& fork);
+// row_meta of a second pass: the degrees stay, no entry counts as pruned
+void launch_clear_clean(uint32_t* row_meta, uint64_t n, cudaStream_t st);
+// |x|^2 of every row (integer data)
+void launch_row_norms(const IndexView& ix, int* norms, cudaStream_t st);
 
 struct QueryArgs {
   const uint8_t* queries;  // device rows, stride qstride (zero padded to 16 bytes)

@@ -49,15 +49,81 @@ __device__ __forceinline__ PruneSmem prune_ws(uint32_t* cid, float* ckey, uint8_
   return p;
 }
 
-// One Hoare partition of [first, last) around the pivot at `pivot` (= first-1),
-// done by the warp: the k-th "not less" position from the left is swapped
-// with the k-th "not greater" position from the right for every k where the
-// former is left of the latter (ddsort::partition_by_rank_pairing).
-__device__ __forceinline__ int warp_partition_rank(const ddsort::Arr<uint32_t>& A, int first,
-                                                   int last, int pivot, int* posL, int* posR) {
+// One Hoare partition of [first, last) around the pivot value pk held at
+// first - 1, done by the warp with one element per lane and word (n = last -
+// first <= 32 W), the stops kept as ballot words.  Rank pairing
+// (ddsort::partition_by_rank_pairing) swaps the k-th "not less" position from
+// the left (l_k) with the k-th "not greater" one from the right (r_k) while
+// l_k < r_k.  With a(x) left stops before x and b(x) right stops from x on,
+// pair k is swapped iff some x has a(x) >= k and b(x) >= k, so the number of
+// pairs is K = max over x of min(a(x), b(x)): no list of stops is written or
+// searched.  The elements of the K pairs change places through exi / exk (2K
+// <= n entries); the return value min(l_{K+1}, r_K) is a minimum over lanes.
+// A list that says nothing about its stops (NaN keys) returns `last`, which
+// the caller's depth budget ends.
+template <int W>
+__device__ __forceinline__ int warp_partition_words(const ddsort::Arr<uint32_t>& A, int first,
+                                                    int last, float pk, int* exi, float* exk) {
   const uint32_t FULL = 0xffffffffu;
   const int lane = (int)lane_id();
-  const float pk = A.key[pivot];
+  const uint32_t lt = lanemask_lt_();
+  float key[W];
+  uint32_t Lw[W], Rw[W];
+  int totR = 0;
+#pragma unroll
+  for (int t = 0; t < W; t++) {
+    const int p = first + lane + 32 * t;
+    const bool in = p < last;
+    key[t] = in ? A.key[p] : 0.f;
+    Lw[t] = __ballot_sync(FULL, in && !(key[t] < pk));
+    Rw[t] = __ballot_sync(FULL, in && !(pk < key[t]));
+    totR += __popc(Rw[t]);
+  }
+  int rl[W], rr[W];  // left stops before, right stops from this position on
+  int pl = 0, pr = 0, kk = 0;
+#pragma unroll
+  for (int t = 0; t < W; t++) {
+    rl[t] = pl + __popc(Lw[t] & lt);
+    rr[t] = totR - pr - __popc(Rw[t] & lt);
+    kk = max(kk, min(rl[t], rr[t]));
+    pl += __popc(Lw[t]);
+    pr += __popc(Rw[t]);
+  }
+  const int K = (int)__reduce_max_sync(FULL, (uint32_t)kk);
+  int c = last;
+  bool sl[W], sr[W];
+#pragma unroll
+  for (int t = 0; t < W; t++) {
+    const int p = first + lane + 32 * t;
+    const bool isL = (Lw[t] >> lane) & 1u, isR = (Rw[t] >> lane) & 1u;
+    rr[t] -= 1;  // 0-based rank from the right when this position is a right stop
+    sl[t] = isL && rl[t] < K;
+    sr[t] = isR && rr[t] < K;
+    if ((isL && rl[t] == K) || (isR && rr[t] == K - 1)) c = min(c, p);
+    if (sl[t] || sr[t]) {
+      const int dst = sl[t] ? rl[t] : K + rr[t];
+      exi[dst] = (int)A.id[p];
+      exk[dst] = key[t];
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < W; t++)
+    if (sl[t] || sr[t]) {
+      const int p = first + lane + 32 * t;
+      const int src = sl[t] ? K + rl[t] : rr[t];
+      A.id[p] = (uint32_t)exi[src];
+      A.key[p] = exk[src];
+    }
+  __syncwarp();
+  return (int)__reduce_min_sync(FULL, (uint32_t)c);
+}
+
+// The same for ranges of any length, the stops listed in posL / posR.
+static __device__ __noinline__ int warp_partition_rank(const ddsort::Arr<uint32_t> A, int first,
+                                                int last, float pk, int* posL, int* posR) {
+  const uint32_t FULL = 0xffffffffu;
+  const int lane = (int)lane_id();
   int nL = 0;
   for (int base = first; base < last; base += 32) {
     const int i = base + lane;
@@ -67,9 +133,9 @@ __device__ __forceinline__ int warp_partition_rank(const ddsort::Arr<uint32_t>& 
     nL += __popc(b);
   }
   int nR = 0;
-  for (int base = last - 1; base >= pivot; base -= 32) {
+  for (int base = last - 1; base >= first; base -= 32) {
     const int i = base - lane;
-    const bool f = i >= pivot && !(pk < A.key[i]);
+    const bool f = i >= first && !(pk < A.key[i]);
     const uint32_t b = __ballot_sync(FULL, f);
     if (f) posR[nR + __popc(b & lanemask_lt_())] = i;
     nR += __popc(b);
@@ -85,18 +151,19 @@ __device__ __forceinline__ int warp_partition_rank(const ddsort::Arr<uint32_t>& 
   }
   for (int k = lane; k < K; k += 32) A.swap(posL[k], posR[k]);
   __syncwarp();
-  if (K == 0) return posL[0];
   const int a = K < nL ? posL[K] : last;
-  const int r = posR[K - 1];
-  return a < r ? a : r;
+  return K == 0 ? a : min(a, posR[K - 1]);
 }
 
 // The introsort partition phase of one range [first0, last0) with the
-// remaining depth budget depth0, replayed by a warp: median-of-three and the
-// heap fallback on lane 0, each partition in parallel; leaf starts are marked
-// in `bits` (atomically when other warps mark neighbouring ranges).  posL /
-// posR need room for last0 - first0 entries; the stack for
-// 3 * (depth0 + 2) ints.
+// remaining depth budget depth0, replayed by a warp: the median of three read
+// by every lane, each partition in parallel (ranges of up to 256 elements as
+// ballot words), the heap fallback on lane 0; leaf starts are marked in `bits`
+// (atomically when other warps mark neighbouring ranges).  posL / posR need
+// room for last0 - first0 entries; the stack for 3 * (depth0 + 2) ints.
+// MAXM: the longest list the caller has (0: any), which leaves out the code
+// for ranges that cannot occur.
+template <int MAXM = 0>
 __device__ __forceinline__ void warp_partition_loop(const ddsort::Arr<uint32_t>& A, int first0,
                                                     int last0, int depth0, int* stack,
                                                     uint32_t* bits, int* posL, int* posR,
@@ -120,10 +187,24 @@ __device__ __forceinline__ void warp_partition_loop(const ddsort::Arr<uint32_t>&
         break;
       }
       --depth;
+      // ddsort::move_median_to_first(first, first + 1, mid, last - 1)
       const int mid = first + (last - first) / 2;
-      if (lane == 0) ddsort::move_median_to_first(A, first, first + 1, mid, last - 1);
+      const float ka = A.key[first + 1], kb = A.key[mid], kc = A.key[last - 1];
+      const int med = ka < kb ? (kb < kc ? mid : (ka < kc ? last - 1 : first + 1))
+                              : (ka < kc ? first + 1 : (kb < kc ? last - 1 : mid));
+      const float pk = med == mid ? kb : (med == first + 1 ? ka : kc);
       __syncwarp();
-      const int cut = warp_partition_rank(A, first + 1, last, first, posL, posR);
+      if (lane == 0) A.swap(first, med);
+      __syncwarp();
+      const int n = last - first - 1;
+      int cut;
+      if (n <= 32)
+        cut = warp_partition_words<1>(A, first + 1, last, pk, posL, (float*)posR);
+      else if (n <= 96 || (MAXM != 0 && MAXM <= 128))
+        cut = warp_partition_words<(MAXM != 0 && MAXM <= 128) ? 4 : 3>(A, first + 1, last, pk, posL,
+                                                                       (float*)posR);
+      else if (n <= 256) cut = warp_partition_words<8>(A, first + 1, last, pk, posL, (float*)posR);
+      else cut = warp_partition_rank(A, first + 1, last, pk, posL, posR);
       if (lane == 0) {
         stack[sp] = cut;
         stack[sp + 1] = last;
@@ -141,55 +222,31 @@ __device__ __forceinline__ void warp_partition_loop(const ddsort::Arr<uint32_t>&
   }
 }
 
-// Fast path of warp_std_sort for lists without equal keys, where std::sort's
-// result is the one ascending order.  Returns false (list untouched) when two
-// keys are equal.  A list already in strictly ascending order is left as is
-// (a sorted list with equal neighbours goes straight back to the caller);
-// otherwise each element's rank (count of smaller keys) is its position, and
-// the list is rewritten through the rank-pairing scratch (2 * cap ints).
-constexpr uint32_t kRankSortMax = 256;
-
-// The rank sort of a list made of one long strictly ascending run and at most
-// 32 other elements: a reverse prune's list, where the target's row is the
-// selection of its last prune (ascending) followed by the few sources
-// appended since, and the new sources come in batch order.  A run element's
-// rank is its place in the run plus the other elements below it; another
-// element's rank is its lower bound in the run (binary search) plus the other
-// elements below it.  Returns 1 when sorted, 0 when two keys are equal (list
-// untouched), -1 when the list does not have that shape (list untouched).
-__device__ __forceinline__ int warp_sort_run_plus_few(const PruneSmem& S, uint32_t m) {
+// A list made of one strictly ascending run [rs, rs + rl) and at most 32 other
+// elements, without equal keys: a reverse prune's list, where the target's row
+// is the selection of its last prune followed by the few sources appended
+// since, and the new sources come in batch order.  std::sort's result is then
+// the one ascending order: a run element's rank is its place in the run plus
+// the other elements below it; another element's rank is its lower bound in
+// the run (binary search) plus the other elements below it.  Returns false,
+// the list untouched, when two keys are equal or the list has another shape.
+__device__ __forceinline__ bool warp_sort_run_plus_few(const PruneSmem& S, uint32_t m, uint32_t rs,
+                                                       uint32_t rl) {
   const uint32_t FULL = 0xffffffffu;
   const uint32_t lane = lane_id();
-  constexpr uint32_t kMaxRuns = 48;
-  // the longest run [rs, rs + rl): runs start at 0 and where a key is not
-  // above its predecessor
-  uint32_t nruns = 0, prev = 0, rs = 0, rl = 0;
-  for (uint32_t b = 0; b < m && nruns <= kMaxRuns; b += 32) {
+  const uint32_t u = m - rl, re = rs + rl;
+  if (u > 32) return false;
+  bool tie = !(S.ckey[rs] == S.ckey[rs]);
+  for (uint32_t b = rs + 1; b < re; b += 32) {
     const uint32_t i = b + lane;
-    const bool st = i < m && i > 0 && !(S.ckey[i - 1] < S.ckey[i]);
-    for (uint32_t bits = __ballot_sync(FULL, st); bits; bits &= bits - 1) {
-      const uint32_t s0 = b + __ffs(bits) - 1;
-      if (s0 - prev > rl) {
-        rl = s0 - prev;
-        rs = prev;
-      }
-      prev = s0;
-      nruns++;
-    }
+    if (i < re && !(S.ckey[i - 1] < S.ckey[i])) tie = true;
   }
-  if (m - prev > rl) {
-    rl = m - prev;
-    rs = prev;
-  }
-  const uint32_t u = m - rl;
-  if (nruns > kMaxRuns || u > 32) return -1;
   // lane q < u holds the q-th element outside the run
   const bool qv = lane < u;
   const uint32_t qi = lane < rs ? lane : lane + rl;
   const float kq = qv ? S.ckey[qi] : 0.f;
-  const uint32_t re = rs + rl;
+  if (__any_sync(FULL, tie || (qv && kq != kq))) return false;
   uint32_t rq = rs;
-  bool tie = false;
   if (qv) {
     uint32_t hi = re;
     while (rq < hi) {
@@ -205,7 +262,7 @@ __device__ __forceinline__ int warp_sort_run_plus_few(const PruneSmem& S, uint32
     rq += kj < kq ? 1u : 0u;
     tie |= qv && j != lane && kj == kq;
   }
-  if (__any_sync(FULL, tie)) return 0;
+  if (__any_sync(FULL, tie)) return false;
   int* tid = S.posL;
   float* tkey = (float*)S.posR;
   if (qv) {
@@ -220,58 +277,6 @@ __device__ __forceinline__ int warp_sort_run_plus_few(const PruneSmem& S, uint32
     if (i < rl) {
       tid[r] = (int)S.cid[rs + i];
       tkey[r] = ki;
-    }
-  }
-  __syncwarp();
-  for (uint32_t i = lane; i < m; i += 32) {
-    S.cid[i] = (uint32_t)tid[i];
-    S.ckey[i] = tkey[i];
-  }
-  __syncwarp();
-  return 1;
-}
-
-__device__ __forceinline__ bool warp_sort_distinct(const PruneSmem& S, uint32_t m) {
-  const uint32_t FULL = 0xffffffffu;
-  const uint32_t lane = lane_id();
-  bool strict = true, nondesc = true;
-  for (uint32_t b = 1; b < m && nondesc; b += 32) {
-    const uint32_t i = b + lane;
-    const float k0 = i < m ? S.ckey[i - 1] : 0.f, k1 = i < m ? S.ckey[i] : 1.f;
-    strict = __all_sync(FULL, !strict ? false : k0 < k1) && strict;
-    nondesc = __all_sync(FULL, k0 <= k1);
-  }
-  if (strict && nondesc) return true;
-  if (nondesc || m > kRankSortMax) return false;
-  const int rp = warp_sort_run_plus_few(S, m);
-  if (rp >= 0) return rp == 1;
-  uint32_t rk[kRankSortMax / 32];
-  bool tie = false;
-#pragma unroll
-  for (int t = 0; t < (int)(kRankSortMax / 32); t++) {
-    const uint32_t i = lane + 32u * t;
-    rk[t] = 0;
-    if (i < m) {
-      const float ki = S.ckey[i];
-      uint32_t r = 0, eq = 0;
-      for (uint32_t j = 0; j < m; j++) {
-        const float kj = S.ckey[j];
-        r += kj < ki ? 1u : 0u;
-        eq += kj == ki ? 1u : 0u;
-      }
-      rk[t] = r;
-      tie |= eq != 1u;
-    }
-  }
-  if (__any_sync(FULL, tie)) return false;
-  int* tid = S.posL;
-  float* tkey = (float*)S.posR;
-#pragma unroll
-  for (int t = 0; t < (int)(kRankSortMax / 32); t++) {
-    const uint32_t i = lane + 32u * t;
-    if (i < m) {
-      tid[rk[t]] = (int)S.cid[i];
-      tkey[rk[t]] = S.ckey[i];
     }
   }
   __syncwarp();
@@ -321,19 +326,32 @@ __device__ __forceinline__ void warp_finish_leaves(const PruneSmem& S, uint32_t 
 }
 
 // Orders cid/ckey[0, m) exactly like std::sort with the distance-only
-// comparator: lists without equal keys take warp_sort_distinct; otherwise
-// the warp replays the partition phase, marking leaf starts in a bitmap, and
-// the leaves are finished in parallel (warp_finish_leaves).
-__device__ __forceinline__ void warp_std_sort(const PruneSmem& S, uint32_t m) {
+// comparator.  A strictly ascending list is left as it is, a list of one
+// ascending run [rs, rs + rl) (rl = 0: none known) and a few other elements
+// without equal keys is ranked from the run, and every other list replays the
+// introsort: the warp replays the partition phase, marking leaf starts in a
+// bitmap, and the leaves are finished in parallel (warp_finish_leaves).
+template <int MAXM = 0>
+__device__ __forceinline__ void warp_std_sort(const PruneSmem& S, uint32_t m, uint32_t rs = 0,
+                                              uint32_t rl = 0) {
   const uint32_t lane = lane_id();
-  if (warp_sort_distinct(S, m)) return;
+  if (rl) {
+    if (warp_sort_run_plus_few(S, m, rs, rl)) return;
+  } else {
+    bool strict = true;
+    for (uint32_t b = 1; b < m && strict; b += 32) {
+      const uint32_t i = b + lane;
+      strict = __all_sync(0xffffffffu, i >= m || S.ckey[i - 1] < S.ckey[i]);
+    }
+    if (strict) return;
+  }
   ddsort::Arr<uint32_t> A{S.cid, S.ckey};
   const uint32_t nw = (m + 31) / 32;
   for (uint32_t w = lane; w < nw; w += 32) S.leafbits[w] = 0;
   __syncwarp();
   if (m > 0)
-    warp_partition_loop(A, 0, (int)m, 2 * ddsort::floor_log2((int)m), S.stack, S.leafbits, S.posL,
-                        S.posR, false);
+    warp_partition_loop<MAXM>(A, 0, (int)m, 2 * ddsort::floor_log2((int)m), S.stack, S.leafbits,
+                              S.posL, S.posR, false);
   warp_finish_leaves(S, m);
 }
 
@@ -344,44 +362,50 @@ __device__ __forceinline__ uint32_t cta_reduce_add(uint32_t v, uint32_t* sh) {
   return tot;
 }
 
-// One Hoare partition (rank pairing) done by the whole CTA; the pivot value
-// must be in place at `pivot` (= first - 1) before the call.
+// One Hoare partition (rank pairing) of [first, last) done by the whole CTA
+// around the pivot value at first - 1, which must be in place before the call.
+// Each warp takes one contiguous piece and reads it 32 elements at a time:
+// once to count its stops, once to list them.
 __device__ __forceinline__ int cta_partition_rank(const ddsort::Arr<uint32_t>& A, int first,
-                                                  int last, int pivot, int* posL, int* posR,
-                                                  uint32_t* sh) {
-  const int NT = (int)blockDim.x, tid = (int)threadIdx.x;
-  const float pk = A.key[pivot];
-  // left stops, ascending: contiguous chunks per thread
-  const int n = last - first;
-  const int ch = (n + NT - 1) / NT;
-  const int lo = first + tid * ch, hi = min(last, lo + ch);
-  uint32_t c = 0;
-  for (int i = lo; i < hi; i++) c += !(A.key[i] < pk) ? 1u : 0u;
-  uint32_t nL;
-  uint32_t j = cta_scan_excl(c, &nL, sh);
-  for (int i = lo; i < hi; i++)
-    if (!(A.key[i] < pk)) posL[j++] = i;
-  // right stops, descending over [pivot, last)
-  const int nr = last - pivot;
-  const int ch2 = (nr + NT - 1) / NT;
-  const int q0 = tid * ch2, q1 = min(nr, q0 + ch2);
-  c = 0;
-  for (int q = q0; q < q1; q++) c += !(pk < A.key[last - 1 - q]) ? 1u : 0u;
-  uint32_t nR;
-  j = cta_scan_excl(c, &nR, sh);
-  for (int q = q0; q < q1; q++)
-    if (!(pk < A.key[last - 1 - q])) posR[j++] = last - 1 - q;
+                                                  int last, int* posL, int* posR, uint32_t* sh) {
+  const uint32_t FULL = 0xffffffffu;
+  const int NT = (int)blockDim.x, tid = (int)threadIdx.x, lane = tid & 31;
+  const float pk = A.key[first - 1];
+  const int nwarps = NT >> 5, w = tid >> 5;
+  const int per = ((last - first + nwarps - 1) / nwarps + 31) & ~31;
+  // left stops, ascending
+  const int lo = min(last, first + w * per), hi = min(last, lo + per);
+  uint32_t cl = 0, cr = 0;
+  for (int b = lo; b < hi; b += 32) {
+    const int i = b + lane;
+    const float k = i < hi ? A.key[i] : 0.f;
+    cl += __popc(__ballot_sync(FULL, i < hi && !(k < pk)));
+    cr += __popc(__ballot_sync(FULL, i < hi && !(pk < k)));
+  }
+  // (exclusive scans over the warps: lane 0 of each carries its count)
+  uint32_t nL, nR;
+  uint32_t ol = __shfl_sync(FULL, cta_scan_excl(lane == 0 ? cl : 0u, &nL, sh), 0);
+  uint32_t orr = __shfl_sync(FULL, cta_scan_excl(lane == 0 ? cr : 0u, &nR, sh), 0);
+  for (int b = lo; b < hi; b += 32) {
+    const int i = b + lane;
+    const float k = i < hi ? A.key[i] : 0.f;
+    const bool fl = i < hi && !(k < pk), fr = i < hi && !(pk < k);
+    const uint32_t bl = __ballot_sync(FULL, fl), br = __ballot_sync(FULL, fr);
+    if (fl) posL[ol + __popc(bl & lanemask_lt_())] = i;
+    if (fr) posR[nR - 1 - (orr + __popc(br & lanemask_lt_()))] = i;  // descending
+    ol += __popc(bl);
+    orr += __popc(br);
+  }
   __syncthreads();
   const int lim = (int)min(nL, nR);
-  c = 0;
+  uint32_t c = 0;
   for (int k = tid; k < lim; k += NT) c += posL[k] < posR[k] ? 1u : 0u;
   const int K = (int)cta_reduce_add(c, sh);  // the pairs with posL < posR form a prefix
   for (int k = tid; k < K; k += NT) A.swap(posL[k], posR[k]);
-  __syncthreads();
-  if (K == 0) return posL[0];
   const int a = K < (int)nL ? posL[K] : last;
-  const int r = posR[K - 1];
-  return a < r ? a : r;
+  const int cut = K == 0 ? a : min(a, posR[K - 1]);
+  __syncthreads();
+  return cut;
 }
 
 // Greedy selection over the sorted candidates; writes the selected ids to
