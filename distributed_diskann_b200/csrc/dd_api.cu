@@ -87,6 +87,8 @@ struct dd_index {
   uint64_t qhash_words = 0;
   uint32_t* qev = nullptr;    // evicted lists of the query searches
   uint64_t qev_words = 0;
+  uint8_t* gtbuf = nullptr;   // ground truth: queries, results and workspace
+  uint64_t gtbuf_bytes = 0;
   // sharded build: the launch shapes and parameters set by dd_shard_begin
   bool shard_ready = false;
   dd_build_params shard_params{};
@@ -199,6 +201,7 @@ int check_error_word(dd_index* h, uint32_t* bits = nullptr) {
     if (e & DD_ECAND_CAP) m += " a per-query beam width was 0, below k or above Lmax;";
     if (e & DD_EDEGREE) m += " row degree exceeds R;";
     if (e & DD_ESEG_CAP) m += " reverse-edge group exceeded the workspace;";
+    if (e & DD_ETIMEOUT) m += " a kernel's wait ran out;";
     return fail(h, DD_ERR_DEVICE, "%s", m.c_str());
   }
   return DD_OK;
@@ -698,6 +701,7 @@ int dd_destroy(dd_index* h) {
   dfree(h->qcls);
   dfree(h->qhash);
   dfree(h->qev);
+  dfree(h->gtbuf);
   if (h->gexec) cudaGraphExecDestroy(h->gexec);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   for (cudaStream_t a : h->fork.aux)
@@ -1526,30 +1530,61 @@ int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   if (nq == 0) return DD_OK;
   CK(cudaSetDevice(h->device));
   uint64_t rb = (uint64_t)h->d * esize(h->dtype), ds = h->stride;
-  uint32_t nchunks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(256, h->n / 4096));
-  uint8_t* dq = nullptr;
-  uint32_t *di = nullptr, *pi = nullptr;
-  float* dd = nullptr;
-  double* pd = nullptr;
-  cudaError_t e = dalloc(&dq, nq * ds);
-  if (e == cudaSuccess) e = dalloc(&di, nq * k);
-  if (e == cudaSuccess) e = dalloc(&dd, nq * k);
-  if (e == cudaSuccess) e = dalloc(&pi, nq * nchunks * k);
-  if (e == cudaSuccess) e = dalloc(&pd, nq * nchunks * k);
+  const IndexView ix = view(h);
+  // one buffer, kept with the handle up to kGtKeepBytes: allocating and freeing
+  // megabytes costs about a millisecond, more than a small call's kernels
+  constexpr uint64_t kGtKeepBytes = 1ull << 30;
+  auto r256 = [](uint64_t x) { return (x + 255) & ~(uint64_t)255; };
+  const uint64_t work_bytes = groundtruth_work_bytes(ix, nq, h->sm_count);
+  const uint64_t need = r256(nq * ds) + 2 * r256(nq * k * 4ull) + work_bytes;
+  if (need > h->gtbuf_bytes) {
+    dfree(h->gtbuf);
+    h->gtbuf = nullptr;
+    h->gtbuf_bytes = 0;
+    CK(dalloc(&h->gtbuf, need));
+    h->gtbuf_bytes = need;
+  }
+  uint8_t* dq = h->gtbuf;
+  uint32_t* di = (uint32_t*)(dq + r256(nq * ds));
+  float* dd = (float*)((uint8_t*)di + r256(nq * k * 4ull));
+  uint8_t* work = (uint8_t*)dd + r256(nq * k * 4ull);
+  uint8_t* parts = nullptr;
+  uint32_t *over = nullptr, nover = 0;
+  bool ok = true;
+  cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = cudaMemsetAsync(dq, 0, nq * ds, h->stream);
   if (e == cudaSuccess)
     e = cudaMemcpy2DAsync(dq, ds, queries, qstride, rb, nq, cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess) {
-    launch_groundtruth(view(h), dq, ds, nq, k, di, dd, pd, pi, nchunks, h->stream);
+    ok = launch_groundtruth(ix, dq, ds, nq, k, di, dd, work, h->sm_count, h->stream, &over);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(ids, di, nq * k * 4, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dists, dd, nq * k * 4, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  void* fr[] = {dq, di, dd, pi, pd};
-  for (void* q : fr) dfree(q);
+  if (ok) {
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(&nover, over, 4, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    // float queries whose candidates the screen could not bound
+    const uint64_t per = (uint64_t)groundtruth_exact_chunks(ix) * k * 12;
+    const uint32_t batch = (uint32_t)std::min<uint64_t>(nover, std::max<uint64_t>(1, (256ull << 20) / per));
+    if (e == cudaSuccess && nover) e = dalloc(&parts, batch * per);
+    for (uint32_t f = 0; e == cudaSuccess && f < nover; f += batch) {
+      launch_groundtruth_exact(ix, dq, ds, nq, f, std::min(batch, nover - f), k, di, dd, work,
+                               h->sm_count, parts, h->stream);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ids, di, nq * k * 4, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dists, dd, nq * k * 4, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  }
+  dfree(parts);
+  if (h->gtbuf_bytes > kGtKeepBytes) {
+    dfree(h->gtbuf);
+    h->gtbuf = nullptr;
+    h->gtbuf_bytes = 0;
+  }
   CK(e);
-  return DD_OK;
+  if (!ok) return fail(h, DD_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+  return check_error_word(h);
 }
 
 // the caller may write the points through this pointer: the BF16 row copies

@@ -20,6 +20,7 @@
 #define DD_ECAND_CAP 0x4u     // a per-query beam width was 0, below k, or above the launch maximum
 #define DD_EDEGREE 0x8u       // a row would exceed R (reference aborts: graph.h:61-93)
 #define DD_ESEG_CAP 0x10u     // reverse-edge segment exceeded its capacity
+#define DD_ETIMEOUT 0x20u     // a kernel's wait for its own copies ran out
 
 enum dd_dtype_e { DD_F32 = 0, DD_I8 = 1, DD_U8 = 2 };
 enum dd_metric_e { DD_L2 = 0, DD_MIPS = 1 };

@@ -246,10 +246,20 @@ struct PruneArgs {
 };
 void launch_prune_tasks(const IndexView& ix, const PruneArgs& pa, cudaStream_t st);
 
-// brute-force ground truth (FP64 for float data, exact integers otherwise)
-void launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qstride, uint64_t nq,
-                        uint32_t k, uint32_t* ids, float* dists, double* part_d,
-                        uint32_t* part_i, uint32_t nchunks, cudaStream_t st);
+// brute-force ground truth (k_gt.cu): device queries of stride qstride (a
+// multiple of 64, zero padded), a workspace of groundtruth_work_bytes; *over
+// names the device word that says how many float queries
+// launch_groundtruth_exact must still compute.  False: no tensor map could be
+// made.
+uint64_t groundtruth_work_bytes(const IndexView& ix, uint64_t nq, int sm_count);
+bool launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qstride, uint64_t nq,
+                        uint32_t k, uint32_t* ids, float* dists, uint8_t* work, int sm_count,
+                        cudaStream_t st, uint32_t** over);
+uint32_t groundtruth_exact_chunks(const IndexView& ix);
+void launch_groundtruth_exact(const IndexView& ix, const uint8_t* queries, uint64_t qstride,
+                              uint64_t nq, uint32_t first, uint32_t count, uint32_t k,
+                              uint32_t* ids, float* dists, const uint8_t* work, int sm_count,
+                              uint8_t* parts, cudaStream_t st);
 
 // sharded build exchange: the rows of the targets this rank's reverse step
 // changed (segments of the grouped pairs, st/heads/counters as in
