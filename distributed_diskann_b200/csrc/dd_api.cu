@@ -468,7 +468,10 @@ int grid_for(const LaunchPlan& pl, uint64_t B, int sm_count) {
 int tune_round(dd_index* h, RoundArgs ra, BuildPlan* bp, TuneResult* res) {
   IndexView ix = view(h);
   if (bp->screen) attach_screen(h, &ix);
-  if (bp->fast) ix.fgroup_lg = fast_fgroup(h);
+  if (bp->fast) {
+    ix.fgroup_lg = fast_fgroup(h);
+    ix.norms = h->norms;
+  }
   ra.B = std::min<uint32_t>(ra.B, kTuneItems);
   cudaEvent_t a, b;
   CK(cudaEventCreate(&a));
@@ -916,7 +919,7 @@ int build_once(dd_index* h, const dd_build_params* P, uint32_t vcap, dd_stats* s
   BuildPlan bp;
   bp.fast = P->mode == DD_MODE_FAST;
   const bool fastf = bp.fast && use_h24(h) && rows_without_repeats(h, P);
-  bp.slay = make_search_layout(h->d, h->dtype, P->L, h->Rp, vcap, true, use_h24(h), true, fastf);
+  bp.slay = make_search_layout(h->d, h->dtype, h->metric, P->L, h->Rp, vcap, true, use_h24(h), true, fastf);
   if (bp.slay.total > 227 * 1024)
     return fail(h, DD_ERR_UNSUPPORTED, "per-warp shared memory %u B too large (L=%u)",
                 bp.slay.total, P->L);
@@ -1111,7 +1114,7 @@ BuildPlan shard_plan(dd_index* h) {
   BuildPlan bp;
   bp.fast = P->mode == DD_MODE_FAST;
   const bool fastf = bp.fast && use_h24(h) && rows_without_repeats(h, P);
-  bp.slay = make_search_layout(h->d, h->dtype, P->L, h->Rp, vcap, true, use_h24(h), true, fastf);
+  bp.slay = make_search_layout(h->d, h->dtype, h->metric, P->L, h->Rp, vcap, true, use_h24(h), true, fastf);
   bp.play = make_prune_layout(h->d, h->dtype, h->Rp, bp.slay.ccap, bp.fast);
   bp.splan = plan_search(view(h), bp.slay, P->L);
   bp.pplan = plan_prune(view(h), bp.play, bp.fast);
@@ -1167,6 +1170,7 @@ int dd_shard_begin(dd_index* h, const dd_build_params* P, uint64_t max_batch) {
     rc = ensure_screen(h);
     if (rc) return rc;
   }
+  if (bp.fast && !h->norms && greedy_uses_mma(h->d, h->dtype)) CK(dalloc(&h->norms, h->n));
   CK(cudaMemsetAsync(h->graph, 0xff, h->n * h->Rp * 4ull, h->stream));
   CK(cudaMemsetAsync(h->err, 0, 4, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -1195,7 +1199,11 @@ int dd_shard_search_prune(dd_index* h, uint64_t lo, uint64_t hi, uint32_t* rows)
     if (rc) return rc;
     attach_screen(h, &ix);
   }
-  if (bp.fast) ix.fgroup_lg = fast_fgroup(h);
+  if (bp.fast) {
+    ix.fgroup_lg = fast_fgroup(h);
+    if (h->norms) launch_row_norms(ix, h->norms, h->stream);  // the points may have changed
+    ix.norms = h->norms;
+  }
   launch_search(ix, ra, bp.slay, bp.splan, grid_for(bp.splan, ra.B, h->sm_count), h->stream);
   launch_prune_round(ix, ra, bp.play, bp.slay.vcap, bp.pplan, grid_for(bp.pplan, ra.B, h->sm_count),
                      bp.fast, h->stream);
@@ -1258,7 +1266,7 @@ int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   if (qstride % 16) return fail(h, DD_ERR_ARG, "device query stride must be a multiple of 16");
   CK(cudaSetDevice(h->device));
   h->launches = 0;
-  WarpLayout lay = make_search_layout(h->d, h->dtype, Lmax, h->Rp, 2 * Lmax + 64, false,
+  WarpLayout lay = make_search_layout(h->d, h->dtype, h->metric, Lmax, h->Rp, 2 * Lmax + 64, false,
                                       use_h24(h), false);
   if ((size_t)lay.total > 227 * 1024)
     return fail(h, DD_ERR_UNSUPPORTED, "query shared memory %u B too large", lay.total);
@@ -1344,7 +1352,7 @@ int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
     // seen tables above 16 KB (beam widths above 128) would cap the resident
     // queries per SM by shared memory: they go to one global slice per warp
     const bool hglob = hash_table_bytes(hash_bits_for(Lc), use_h24(h)) > 16384;
-    WarpLayout lc = make_search_layout(h->d, h->dtype, Lc, h->Rp, 2 * Lc + 64, false,
+    WarpLayout lc = make_search_layout(h->d, h->dtype, h->metric, Lc, h->Rp, 2 * Lc + 64, false,
                                        use_h24(h), false, false, hglob);
     const LaunchPlan plan = plan_query(view(h), lc, Lc);
     QueryArgs qc = qa;
@@ -1428,7 +1436,7 @@ int dd_beam_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   if (start >= h->n) return fail(h, DD_ERR_ARG, "start point >= n");
   CK(cudaSetDevice(h->device));
   uint64_t rb = (uint64_t)h->d * esize(h->dtype), ds = h->stride;
-  WarpLayout lay = make_search_layout(h->d, h->dtype, L, h->Rp, vcap, false, use_h24(h));
+  WarpLayout lay = make_search_layout(h->d, h->dtype, h->metric, L, h->Rp, vcap, false, use_h24(h));
   if (lay.total > 227 * 1024) return fail(h, DD_ERR_UNSUPPORTED, "beam shared memory too large");
   const int bgrid = (int)std::min<uint64_t>(nq, 4096);
   uint8_t* dq = nullptr;

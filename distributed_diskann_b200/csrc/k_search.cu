@@ -23,18 +23,21 @@ namespace ddk {
 //   query / debug: qv | frontier | step candidates | visited | evicted | hash.
 // With h24 the hash table stores 24-bit ids (3 bytes a slot instead of 4),
 // which is exact whenever every id is below 0xFFFFFF.
-WarpLayout make_search_layout(uint32_t d, int dtype, uint32_t L, uint32_t Rp, uint32_t vcap,
-                              bool build, bool h24, bool keep_vis, bool fastf, bool hash_global) {
+WarpLayout make_search_layout(uint32_t d, int dtype, int metric, uint32_t L, uint32_t Rp,
+                              uint32_t vcap, bool build, bool h24, bool keep_vis, bool fastf, bool hash_global) {
   WarpLayout w{};
   uint32_t esz = dtype == DD_F32 ? 4 : 1;
   uint32_t off = 0;
   w.qv = off; off += r16((uint64_t)d * esz);
-  w.fr_id = off; off += r16(4ull * L);
-  w.fr_d = off; off += r16(4ull * L);
+  // the fast build search keeps one 64-bit key per entry of a padded frontier
+  w.nf = (build && fastf && L <= 128) ? (L <= 64 ? 64 : 128) : 0;
+  w.fr_id = off; off += r16(w.nf ? 8ull * w.nf : 4ull * L);
+  w.fr_d = off; off += r16(w.nf ? 0 : 4ull * L);
   w.c_id = off; off += r16(4ull * Rp);
   w.c_d = off; off += r16(4ull * Rp);
   w.s_id = off; off += r16(4ull * Rp);
-  w.s_d = off; off += r16(4ull * Rp);
+  w.s_d = off; off += w.nf ? 0 : r16(4ull * Rp);
+  w.term = off; off += w.nf && dtype == DD_F32 && metric == DD_L2 ? kFloatTermBytes : 0;
   w.vcap = vcap;
   w.ccap = vcap + Rp;
   w.fastf = (build && fastf) ? 1u : 0u;
@@ -64,6 +67,19 @@ WarpLayout make_search_layout(uint32_t d, int dtype, uint32_t L, uint32_t Rp, ui
   return w;
 }
 
+// |query|^2 of a staged integer query (16-byte words, zero padded), every lane
+template <int DT>
+__device__ __forceinline__ int query_norm(const uint8_t* qv, uint32_t d) {
+  if (DT == DD_F32) return 0;
+  const uint32_t lane = lane_id();
+  uint32_t s = 0;
+  if (lane < (d + 3) / 4) {
+    const uint32_t v = ((const uint32_t*)qv)[lane];
+    s = DT == DD_U8 ? __dp4a(v, v, 0u) : (uint32_t)__dp4a((int)v, (int)v, 0);
+  }
+  return (int)__reduce_add_sync(0xffffffffu, s);
+}
+
 // build search: visited list in the global slice vis_g (vcap ids then vcap dists)
 __device__ __forceinline__ SearchSmem carve_build(uint8_t* base, const WarpLayout& w, uint32_t* vis_g) {
   SearchSmem S;
@@ -80,6 +96,7 @@ __device__ __forceinline__ SearchSmem carve_build(uint8_t* base, const WarpLayou
   S.ev_bloom = nullptr;
   S.hash = (uint32_t*)(base + w.ws);
   S.h24 = (int)w.h24;
+  S.term = (float*)(base + w.term);
   return S;
 }
 
@@ -104,6 +121,7 @@ __device__ __forceinline__ SearchSmem carve_query(uint8_t* base, const WarpLayou
   S.hash = w.hash_global ? global_hash
                          : (uint32_t*)(base + w.ws + 128 + (w.keep_vis ? r16(4ull * w.vcap) : 0));
   S.h24 = (int)w.h24;
+  S.term = (float*)(base + w.term);
   return S;
 }
 
@@ -111,12 +129,20 @@ __device__ __forceinline__ SearchSmem carve_query(uint8_t* base, const WarpLayou
 // k_search: one warp per batch point runs beam_search on the round-start graph
 // and leaves its visited list in the point's global slice
 // (include/index.h:274-278; src/bsp_index.hpp:259-268).
-// FASTF: the fast form's seen filter, with registers capped at 64 (L <= 128)
-// so that four CTAs of up to 8 warps fit an SM; at L = 128 a search takes
-// 6.2 KB of shared memory with that filter's 4 KB table, and the autotuner
-// settles on four 7-warp CTAs (28 searches per SM).
+// FASTF: the fast form's seen filter and, for L <= 128, warp_build_search with
+// capped registers.  Integer data: 64, so that four CTAs of up to 8 warps fit an
+// SM (4M x 128 uint8 searches 374 ms, with 72 registers 380, with 80 401);
+// float L2: 72, four CTAs of 7 warps (100k x 64: 8.26 ms, 64 registers 8.52);
+// float inner product: 80, three CTAs of 8 warps (400k x 200: 98.6 ms, 64
+// registers 100.4).
+template <int DT, int MT>
+struct SearchBounds {
+  static constexpr int threads = DT == DD_F32 && MT == DD_L2 ? 224 : 256;
+  static constexpr int ctas = DT == DD_F32 && MT == DD_MIPS ? 3 : 4;
+};
 template <int DT, int MT, int FPL, int CPL, bool FASTF>
-__global__ void __launch_bounds__((FASTF && FPL == 4) ? 256 : 512, (FASTF && FPL == 4) ? 4 : 1)
+__global__ void __launch_bounds__((FASTF && FPL == 4) ? SearchBounds<DT, MT>::threads : 512,
+                                  (FASTF && FPL == 4) ? SearchBounds<DT, MT>::ctas : 1)
     k_search(IndexView ix, RoundArgs ra, WarpLayout lay) {
   extern __shared__ uint4 smem_raw[];
   const uint32_t wpc = blockDim.x >> 5;
@@ -124,21 +150,27 @@ __global__ void __launch_bounds__((FASTF && FPL == 4) ? 256 : 512, (FASTF && FPL
   const uint64_t gw = (uint64_t)blockIdx.x * wpc + wic;
   uint8_t* base = (uint8_t*)smem_raw + (size_t)wic * lay.total;
   SearchParams P;
-  P.points = ix.points; P.stride = ix.stride; P.graph = ix.graph; P.Rp = ix.Rp; P.n = ix.n;
+  P.points = ix.points; P.stride = (uint32_t)ix.stride; P.graph = ix.graph; P.Rp = ix.Rp; P.n = ix.n;
   P.d = ix.d; P.start = ra.start; P.L = ra.L; P.k = 0; P.cut = 0.0; P.limit = ix.n;
   P.degree_limit = ix.R; P.hbits = lay.hbits; P.vcap = lay.vcap; P.ecap = 0; P.query_mode = 0;
   P.keep_visited = 1; P.err = ix.err;
-  P.screen = ix.screen; P.sstride = ix.sstride; P.snorm = ix.snorm; P.fgroup_lg = ix.fgroup_lg;
+  P.screen = ix.screen; P.sstride = ix.sstride; P.snorm = ix.snorm; P.fgroup_lg = ix.fgroup_lg; P.norms = ix.norms;
   const uint32_t qb = r16((uint64_t)ix.d * ElemSize<DT>::v);
   uint64_t cur = gw;
   const uint64_t step = (uint64_t)gridDim.x * wpc;
   for (uint64_t b = warp_next_item(ra.qsearch, cur, step); b < ra.B;
        b = warp_next_item(ra.qsearch, cur, step)) {
     const uint32_t p = (uint32_t)(ra.floor + b);
-    const SearchSmem S = carve_build(base, lay, ra.vis_all + b * 2ull * lay.vcap);
+    SearchSmem S = carve_build(base, lay, ra.vis_all + b * 2ull * lay.vcap);
     load_vec(S.qv, ix.points + (uint64_t)p * ix.stride, qb);
     __syncwarp();
-    const SearchOut o = warp_beam_search<DT, MT, FPL, CPL, FASTF>(P, S, p);
+    if (FASTF && FPL == 4) S.qn = query_norm<DT>(S.qv, ix.d);
+    SearchOut o;
+    if (FASTF && FPL == 4)
+      o = lay.nf == 64 ? warp_build_search<DT, MT, 2, CPL>(P, S, p)
+                       : warp_build_search<DT, MT, 4, CPL>(P, S, p);
+    else
+      o = warp_beam_search<DT, MT, FPL, CPL, FASTF>(P, S, p);
     if (lane_id() == 0) {
       ra.stat_vis[b] = o.vis_n;
       if (ra.stat_cmps) ra.stat_cmps[b] = o.cmps;
@@ -171,12 +203,12 @@ __global__ void __launch_bounds__(512) k_query(IndexView ix, QueryArgs qa, WarpL
       if (lane == 0) dd_set_error(ix.err, DD_ECAND_CAP);
       Lq = qa.Lvalid;
     }
-    P.points = ix.points; P.stride = ix.stride; P.graph = ix.graph; P.Rp = ix.Rp; P.n = ix.n;
+    P.points = ix.points; P.stride = (uint32_t)ix.stride; P.graph = ix.graph; P.Rp = ix.Rp; P.n = ix.n;
     P.d = ix.d; P.start = qa.start; P.L = Lq; P.k = qa.k; P.cut = qa.cut; P.limit = qa.limit;
     P.degree_limit = qa.degree_limit; P.hbits = hash_bits_for(P.L); P.vcap = 0;
     P.ecap = qa.ev_cap; P.query_mode = 1; P.keep_visited = 0; P.err = ix.err;
     P.screen = ix.screen; P.sstride = ix.sstride; P.snorm = ix.snorm;
-    P.fgroup_lg = ix.fgroup_lg;
+    P.fgroup_lg = ix.fgroup_lg; P.norms = ix.norms;
     load_vec(S.qv, qa.queries + q * qa.qstride, qb);
     __syncwarp();
     SearchOut o = warp_beam_search<DT, MT, FPL, CPL>(P, S, qa.skip_self ? q : (uint64_t)-1);
@@ -218,11 +250,11 @@ __global__ void __launch_bounds__(32) k_beam(IndexView ix, BeamArgs ba, WarpLayo
   const uint32_t qb = r16((uint64_t)ix.d * ElemSize<DT>::v);
   for (uint64_t q = blockIdx.x; q < ba.nq; q += gridDim.x) {
     SearchParams P;
-    P.points = ix.points; P.stride = ix.stride; P.graph = ix.graph; P.Rp = ix.Rp; P.n = ix.n;
+    P.points = ix.points; P.stride = (uint32_t)ix.stride; P.graph = ix.graph; P.Rp = ix.Rp; P.n = ix.n;
     P.d = ix.d; P.start = ba.start; P.L = ba.L; P.k = ba.k; P.cut = ba.cut; P.limit = ba.limit;
     P.degree_limit = ba.degree_limit; P.hbits = lay.hbits; P.vcap = lay.vcap; P.ecap = lay.vcap;
     P.query_mode = ba.k > 0; P.keep_visited = 1; P.err = ix.err;
-    P.screen = nullptr; P.sstride = 0; P.snorm = nullptr; P.fgroup_lg = 0;  // the plain form
+    P.screen = nullptr; P.sstride = 0; P.snorm = nullptr; P.fgroup_lg = 0; P.norms = nullptr;  // the plain form
     load_vec(S.qv, ba.queries + q * ba.qstride, qb);
     __syncwarp();
     SearchOut o = warp_beam_search<DT, MT, 16, 4>(P, S, (uint64_t)ba.self_ids[q]);

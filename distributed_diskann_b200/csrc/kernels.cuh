@@ -23,6 +23,8 @@ struct WarpLayout {
   uint32_t hash_global;  // query layout: the seen table lives in a global slice per warp
   uint32_t hash_words;   // its size in 32-bit words (16-byte multiple)
   uint32_t ev;           // query layout: evicted list in shared memory (keep_vis layouts)
+  uint32_t term;         // float L2: sums of the distances in progress
+  uint32_t nf;           // fast build search: padded frontier of 64-bit keys (0: id / distance arrays)
 };
 
 // Per-warp shared-memory carve-up of k_prune (byte offsets, 16-byte aligned).
@@ -64,7 +66,7 @@ struct IndexView {
 // fastf (build only): the fast form's seen filter, 16-bit tags (search_core.cuh)
 // hash_global (query only): the seen table goes to a global slice per resident
 // warp (QueryArgs::hash_scratch) instead of shared memory
-WarpLayout make_search_layout(uint32_t d, int dtype, uint32_t L, uint32_t Rp, uint32_t vcap,
+WarpLayout make_search_layout(uint32_t d, int dtype, int metric, uint32_t L, uint32_t Rp, uint32_t vcap,
                               bool build, bool h24, bool keep_vis = true, bool fastf = false,
                               bool hash_global = false);
 // tensor: the fast form's tensor-core greedy (integer data); false: the plain form
