@@ -87,8 +87,13 @@ struct dd_index {
   uint64_t qhash_words = 0;
   uint32_t* qev = nullptr;    // evicted lists of the query searches
   uint64_t qev_words = 0;
-  uint8_t* gtbuf = nullptr;   // ground truth: queries, results and workspace
-  uint64_t gtbuf_bytes = 0;
+  // host calls (search, beam search, prune, ground truth): one device buffer
+  // and one pinned staging buffer, kept up to kIoKeepBytes / kPinKeepBytes
+  uint8_t* io = nullptr;
+  uint64_t io_bytes = 0;
+  uint8_t* pin = nullptr;
+  uint64_t pin_bytes = 0;
+  std::vector<std::pair<uint64_t, LaunchPlan>> qplans;  // query CTA shapes by layout
   // sharded build: the launch shapes and parameters set by dd_shard_begin
   bool shard_ready = false;
   dd_build_params shard_params{};
@@ -172,6 +177,68 @@ cudaError_t dalloc(T** p, uint64_t count) {
 
 void dfree(void* p) {
   if (p) cudaFree(p);
+}
+
+// The buffers of one host call.  Allocating and freeing device memory in every
+// call cost 70 us (small calls) to several ms (megabytes, and cudaFree waits for
+// the device), and each copy from or to pageable memory 15 us or more: the
+// device buffer stays with the handle, the inputs go up in one copy from pinned
+// staging and the results come down in one (up to kPinKeepBytes; larger calls
+// copy each array directly).  512 robustPrune tasks 2.4 -> 0.7 ms, one query 450
+// -> 400 us, 30,000 queries of 100 bytes 18 -> 9.6 ms.
+constexpr uint64_t kIoKeepBytes = 1ull << 30, kPinKeepBytes = 64ull << 20;
+
+struct IoParts {  // byte offsets, 256-byte aligned
+  uint64_t total = 0;
+  uint64_t take(uint64_t bytes) {
+    const uint64_t o = total;
+    total += (bytes + 255) & ~(uint64_t)255;
+    return o;
+  }
+};
+
+int ensure_io(dd_index* h, uint64_t bytes) {
+  if (bytes <= h->io_bytes) return DD_OK;
+  dfree(h->io);
+  h->io = nullptr;
+  h->io_bytes = 0;
+  CK(dalloc(&h->io, bytes));
+  h->io_bytes = bytes;
+  return DD_OK;
+}
+
+// pinned staging of at least `bytes`; null when the call is too large for it
+uint8_t* pinned(dd_index* h, uint64_t bytes) {
+  if (bytes > kPinKeepBytes) return nullptr;
+  if (bytes > h->pin_bytes) {
+    if (h->pin) cudaFreeHost(h->pin);
+    h->pin = nullptr;
+    h->pin_bytes = 0;
+    const uint64_t want = std::max<uint64_t>(bytes, 1u << 20);
+    if (cudaMallocHost((void**)&h->pin, want) != cudaSuccess) {
+      cudaGetLastError();
+      h->pin = nullptr;
+      return nullptr;
+    }
+    h->pin_bytes = want;
+  }
+  return h->pin;
+}
+
+void release_io(dd_index* h) {
+  if (h->io_bytes <= kIoKeepBytes) return;
+  dfree(h->io);
+  h->io = nullptr;
+  h->io_bytes = 0;
+}
+
+// nq rows of rb bytes, qstride apart, into rows of ds bytes (zero padded) at dst
+void stage_rows(uint8_t* dst, uint64_t ds, const uint8_t* src, uint64_t qstride, uint64_t rb,
+                uint64_t nq) {
+  for (uint64_t i = 0; i < nq; i++) {
+    std::memcpy(dst + i * ds, src + i * qstride, rb);
+    std::memset(dst + i * ds + rb, 0, ds - rb);
+  }
 }
 
 // Makes the BF16 row copies current (stream-ordered after the points' upload).
@@ -704,7 +771,8 @@ int dd_destroy(dd_index* h) {
   dfree(h->qcls);
   dfree(h->qhash);
   dfree(h->qev);
-  dfree(h->gtbuf);
+  dfree(h->io);
+  if (h->pin) cudaFreeHost(h->pin);
   if (h->gexec) cudaGraphExecDestroy(h->gexec);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   for (cudaStream_t a : h->fork.aux)
@@ -1254,10 +1322,27 @@ int dd_shard_set_rows(dd_index* h, const uint32_t* ids, const uint32_t* rows, ui
   return check_error_word(h);
 }
 
-int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
+namespace {
+
+// plan_query asks the runtime about eight CTA sizes; the answer depends only on
+// the kernel and its shared memory
+LaunchPlan query_plan(dd_index* h, const WarpLayout& lay, uint32_t L) {
+  const uint64_t key = ((uint64_t)lay.total << 16) | L;
+  for (auto& e : h->qplans)
+    if (e.first == key) return e.second;
+  const LaunchPlan p = plan_query(view(h), lay, L);
+  if (h->qplans.size() >= 64) h->qplans.clear();
+  h->qplans.push_back({key, p});
+  return p;
+}
+
+// dd_search_device; classes: the beam-width classes that may hold a query (bit
+// per class; all when the widths are only known on the device)
+int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
                      const uint32_t* L_per_query, uint32_t Lmax, uint32_t k, double cut,
                      uint64_t limit, uint32_t degree_limit, uint32_t start, int skip_self,
-                     uint32_t* ids, float* dists, uint32_t* visited, uint32_t* cmps) {
+                     uint32_t* ids, float* dists, uint32_t* visited, uint32_t* cmps,
+                     uint32_t classes) {
   if (!h || !queries || !L_per_query || !ids || !dists) return DD_ERR_ARG;
   if (nq == 0) return DD_OK;
   if (Lmax == 0 || Lmax > kMaxL) return fail(h, DD_ERR_UNSUPPORTED, "L must be in [1, %u]", kMaxL);
@@ -1311,7 +1396,7 @@ int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   };
   if (h->search_mode == DD_MODE_PLAIN) {
     // one launch laid out for the largest beam width
-    const LaunchPlan plan = plan_query(view(h), lay, Lmax);
+    const LaunchPlan plan = query_plan(h, lay, Lmax);
     const int wpc = plan.warps_per_cta;
     const int grid = (int)std::min<uint64_t>((nq + wpc - 1) / wpc,
                                              (uint64_t)plan.blocks_per_sm * h->sm_count);
@@ -1344,9 +1429,15 @@ int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   }
   ixq.fgroup_lg = fast_fgroup(h);
   CK(cudaMemsetAsync(counts, 0, 2 * kQueryClasses * 4, h->stream));
-  launch_bin_queries(L_per_query, nq, k, Lmax, h->qcls, counts, h->stream);
-  h->launches = 1;
+  // one class: every query is its, no list needed
+  const bool one = (classes & (classes - 1)) == 0;
+  h->launches = 0;
+  if (!one) {
+    launch_bin_queries(L_per_query, nq, k, Lmax, h->qcls, counts, h->stream);
+    h->launches++;
+  }
   for (int c = query_class(Lmax); c >= 0; c--) {
+    if (!((classes >> c) & 1u)) continue;
     if ((16u << c) < k && c < query_class(Lmax)) break;  // no valid beam width below k
     const uint32_t Lc = std::min<uint32_t>(16u << c, Lmax);
     // seen tables above 16 KB (beam widths above 128) would cap the resident
@@ -1354,11 +1445,11 @@ int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
     const bool hglob = hash_table_bytes(hash_bits_for(Lc), use_h24(h)) > 16384;
     WarpLayout lc = make_search_layout(h->d, h->dtype, h->metric, Lc, h->Rp, 2 * Lc + 64, false,
                                        use_h24(h), false, false, hglob);
-    const LaunchPlan plan = plan_query(view(h), lc, Lc);
+    const LaunchPlan plan = query_plan(h, lc, Lc);
     QueryArgs qc = qa;
     qc.Lmax = Lc;
-    qc.cls_items = h->qcls + (uint64_t)c * nq;
-    qc.cls_count = counts + c;
+    qc.cls_items = one ? nullptr : h->qcls + (uint64_t)c * nq;
+    qc.cls_count = one ? nullptr : counts + c;
     qc.cls_queue = queues + c;
     const int wpc = plan.warps_per_cta;
     const int grid = (int)std::min<uint64_t>((nq + wpc - 1) / wpc,
@@ -1384,6 +1475,16 @@ int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   return DD_OK;
 }
 
+}  // namespace
+
+int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
+                     const uint32_t* L_per_query, uint32_t Lmax, uint32_t k, double cut,
+                     uint64_t limit, uint32_t degree_limit, uint32_t start, int skip_self,
+                     uint32_t* ids, float* dists, uint32_t* visited, uint32_t* cmps) {
+  return search_on_device(h, queries, nq, qstride, L_per_query, Lmax, k, cut, limit, degree_limit,
+                          start, skip_self, ids, dists, visited, cmps, (1u << kQueryClasses) - 1);
+}
+
 int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
               const uint32_t* L_per_query, uint32_t k, double cut, uint64_t limit,
               uint32_t degree_limit, uint32_t start, int skip_self, uint32_t* ids, float* dists,
@@ -1391,39 +1492,56 @@ int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
   if (!h || !queries || !L_per_query || !ids || !dists) return DD_ERR_ARG;
   if (nq == 0) return DD_OK;
   CK(cudaSetDevice(h->device));
-  uint64_t rb = (uint64_t)h->d * esize(h->dtype);
-  uint64_t ds = h->stride;
-  uint32_t Lmax = 0;
+  const uint64_t rb = (uint64_t)h->d * esize(h->dtype), ds = h->stride;
+  uint32_t Lmax = 0, classes = 0;
   for (uint64_t i = 0; i < nq; i++) Lmax = std::max(Lmax, L_per_query[i]);
-  uint8_t* dq = nullptr;
-  uint32_t *dL = nullptr, *di = nullptr, *dv = nullptr, *dc = nullptr;
-  float* dd = nullptr;
-  CK(dalloc(&dq, nq * ds));
-  int rc = DD_OK;
-  cudaError_t e = dalloc(&dL, nq);
-  if (e == cudaSuccess) e = dalloc(&di, nq * k);
-  if (e == cudaSuccess) e = dalloc(&dd, nq * k);
-  if (e == cudaSuccess) e = dalloc(&dv, nq);
-  if (e == cudaSuccess) e = dalloc(&dc, nq);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dq, 0, nq * ds, h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpy2DAsync(dq, ds, queries, qstride, rb, nq, cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dL, L_per_query, nq * 4, cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) {
-    rc = dd_search_device(h, dq, nq, ds, dL, Lmax, k, cut, limit, degree_limit, start, skip_self,
-                          di, dd, dv, dc);
-    if (rc == DD_OK) {
-      e = cudaMemcpyAsync(ids, di, nq * k * 4, cudaMemcpyDeviceToHost, h->stream);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(dists, dd, nq * k * 4, cudaMemcpyDeviceToHost, h->stream);
-      if (e == cudaSuccess && visited) e = cudaMemcpyAsync(visited, dv, nq * 4, cudaMemcpyDeviceToHost, h->stream);
-      if (e == cudaSuccess && cmps) e = cudaMemcpyAsync(cmps, dc, nq * 4, cudaMemcpyDeviceToHost, h->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    }
+  for (uint64_t i = 0; i < nq; i++) {  // an invalid width goes to the class of Lmax (k_bin_queries)
+    const uint32_t L = L_per_query[i];
+    classes |= 1u << query_class(L == 0 || L < k ? Lmax : L);
   }
-  cudaFree(dq); cudaFree(dL); cudaFree(di); cudaFree(dd); cudaFree(dv); cudaFree(dc);
+  IoParts io;
+  const uint64_t o_q = io.take(nq * ds), o_L = io.take(nq * 4), in_bytes = io.total;
+  const uint64_t o_i = io.take(nq * k * 4ull), o_d = io.take(nq * k * 4ull), o_v = io.take(nq * 4),
+                 o_c = io.take(nq * 4), out_bytes = io.total - in_bytes;
+  int rc = ensure_io(h, io.total);
   if (rc) return rc;
+  uint8_t* dev = h->io;
+  uint8_t* pin = pinned(h, std::max(in_bytes, out_bytes));
+  if (pin) {
+    stage_rows(pin + o_q, ds, (const uint8_t*)queries, qstride, rb, nq);
+    std::memcpy(pin + o_L, L_per_query, nq * 4);
+    CK(cudaMemcpyAsync(dev, pin, in_bytes, cudaMemcpyHostToDevice, h->stream));
+  } else {
+    CK(cudaMemsetAsync(dev + o_q, 0, nq * ds, h->stream));
+    CK(cudaMemcpy2DAsync(dev + o_q, ds, queries, qstride, rb, nq, cudaMemcpyHostToDevice, h->stream));
+    CK(cudaMemcpyAsync(dev + o_L, L_per_query, nq * 4, cudaMemcpyHostToDevice, h->stream));
+  }
+  rc = search_on_device(h, dev + o_q, nq, ds, (uint32_t*)(dev + o_L), Lmax, k, cut, limit,
+                        degree_limit, start, skip_self, (uint32_t*)(dev + o_i), (float*)(dev + o_d),
+                        (uint32_t*)(dev + o_v), (uint32_t*)(dev + o_c), classes);
+  cudaError_t e = cudaSuccess;
+  if (rc == DD_OK && pin) {
+    e = cudaMemcpyAsync(pin, dev + in_bytes, out_bytes, cudaMemcpyDeviceToHost, h->stream);
+    rc = e == cudaSuccess ? check_error_word(h) : DD_OK;  // synchronizes
+    const uint8_t* out = pin - in_bytes;
+    if (e == cudaSuccess) {
+      std::memcpy(ids, out + o_i, nq * k * 4ull);
+      std::memcpy(dists, out + o_d, nq * k * 4ull);
+      if (visited) std::memcpy(visited, out + o_v, nq * 4);
+      if (cmps) std::memcpy(cmps, out + o_c, nq * 4);
+    }
+  } else if (rc == DD_OK) {
+    e = cudaMemcpyAsync(ids, dev + o_i, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dists, dev + o_d, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess && visited) e = cudaMemcpyAsync(visited, dev + o_v, nq * 4, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess && cmps) e = cudaMemcpyAsync(cmps, dev + o_c, nq * 4, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess) rc = check_error_word(h);
+  }
+  if (rc || e != cudaSuccess) cudaStreamSynchronize(h->stream);  // the buffers are free again
+  release_io(h);
   CK(e);
-  return check_error_word(h);
+  return rc;
 }
 
 int dd_beam_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
@@ -1439,20 +1557,21 @@ int dd_beam_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   WarpLayout lay = make_search_layout(h->d, h->dtype, h->metric, L, h->Rp, vcap, false, use_h24(h));
   if (lay.total > 227 * 1024) return fail(h, DD_ERR_UNSUPPORTED, "beam shared memory too large");
   const int bgrid = (int)std::min<uint64_t>(nq, 4096);
-  uint8_t* dq = nullptr;
-  int64_t* dself = nullptr;
-  uint32_t *dfi = nullptr, *dfn = nullptr, *dvi = nullptr, *dvn = nullptr, *dcm = nullptr;
-  float *dfd = nullptr, *dvd = nullptr;
-  cudaError_t e = dalloc(&dq, nq * ds);
-  if (e == cudaSuccess) e = dalloc(&dself, nq);
-  if (e == cudaSuccess) e = dalloc(&dfi, nq * L);
-  if (e == cudaSuccess) e = dalloc(&dfd, nq * L);
-  if (e == cudaSuccess) e = dalloc(&dfn, nq);
-  if (e == cudaSuccess) e = dalloc(&dvi, nq * vcap);
-  if (e == cudaSuccess) e = dalloc(&dvd, nq * vcap);
-  if (e == cudaSuccess) e = dalloc(&dvn, nq);
-  if (e == cudaSuccess) e = dalloc(&dcm, nq);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dq, 0, nq * ds, h->stream);
+  IoParts io;
+  const uint64_t o_q = io.take(nq * ds), o_s = io.take(nq * 8), o_fi = io.take(nq * L * 4ull),
+                 o_fd = io.take(nq * L * 4ull), o_fn = io.take(nq * 4),
+                 o_vi = io.take(nq * vcap * 4ull), o_vd = io.take(nq * vcap * 4ull),
+                 o_vn = io.take(nq * 4), o_cm = io.take(nq * 4);
+  int rc = ensure_io(h, io.total);
+  if (rc) return rc;
+  uint8_t* dev = h->io;
+  uint8_t* dq = dev + o_q;
+  int64_t* dself = (int64_t*)(dev + o_s);
+  uint32_t *dfi = (uint32_t*)(dev + o_fi), *dfn = (uint32_t*)(dev + o_fn),
+           *dvi = (uint32_t*)(dev + o_vi), *dvn = (uint32_t*)(dev + o_vn),
+           *dcm = (uint32_t*)(dev + o_cm);
+  float *dfd = (float*)(dev + o_fd), *dvd = (float*)(dev + o_vd);
+  cudaError_t e = cudaMemsetAsync(dq, 0, nq * ds, h->stream);
   if (e == cudaSuccess)
     e = cudaMemcpy2DAsync(dq, ds, queries, qstride, rb, nq, cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(dself, self_ids, nq * 8, cudaMemcpyHostToDevice, h->stream);
@@ -1475,8 +1594,8 @@ int dd_beam_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   if (e == cudaSuccess) e = cudaMemcpyAsync(vis_sizes, dvn, nq * 4, cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(cmps, dcm, nq * 4, cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  void* fr[] = {dq, dself, dfi, dfd, dfn, dvi, dvd, dvn, dcm};
-  for (void* p : fr) dfree(p);
+  if (e != cudaSuccess) cudaStreamSynchronize(h->stream);
+  release_io(h);
   CK(e);
   return check_error_word(h);
 }
@@ -1493,34 +1612,52 @@ int dd_robust_prune(dd_index* h, uint32_t ntasks, const uint32_t* p, const uint6
   CK(cudaSetDevice(h->device));
   uint64_t tot = offsets[ntasks];
   uint64_t ws = tot + (uint64_t)ntasks * h->Rp;
-  uint32_t *dp = nullptr, *dci = nullptr, *dout = nullptr, *gc = nullptr;
-  uint64_t* doff = nullptr;
-  float *dcd = nullptr, *gk = nullptr;
-  int* gl = nullptr;
-  cudaError_t e = dalloc(&dp, ntasks);
-  if (e == cudaSuccess) e = dalloc(&doff, ntasks + 1);
-  if (e == cudaSuccess) e = dalloc(&dci, tot);
-  if (e == cudaSuccess) e = dalloc(&dcd, tot);
-  if (e == cudaSuccess) e = dalloc(&dout, (uint64_t)ntasks * h->Rp);
-  if (e == cudaSuccess) e = dalloc(&gc, ws);
-  if (e == cudaSuccess) e = dalloc(&gk, ws);
-  if (e == cudaSuccess) e = dalloc(&gl, 3 * ws + (uint64_t)ntasks * kGlobalStackInts);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dp, p, ntasks * 4, cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(doff, offsets, (ntasks + 1) * 8ull, cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess && tot) e = cudaMemcpyAsync(dci, cand_ids, tot * 4, cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess && tot) e = cudaMemcpyAsync(dcd, cand_dists, tot * 4, cudaMemcpyHostToDevice, h->stream);
+  uint64_t most = 0;
+  for (uint32_t t = 0; t < ntasks; t++) most = std::max(most, offsets[t + 1] - offsets[t]);
+  IoParts io;
+  const uint64_t o_off = io.take((ntasks + 1) * 8ull), o_p = io.take(ntasks * 4ull),
+                 o_ci = io.take(tot * 4), o_cd = io.take(tot * 4), in_bytes = io.total;
+  const uint64_t o_out = io.take((uint64_t)ntasks * h->Rp * 4), out_bytes = io.total - in_bytes;
+  // lists too long for shared memory keep their workspace in global memory
+  // (the shared form's integer thresholds want an ordinary positive alpha)
+  const bool global = !(alpha > 1e-3 && alpha < 1e3) || !prune_tasks_in_shared(view(h), most);
+  const uint64_t o_gc = io.take(global ? ws * 4 : 0), o_gk = io.take(global ? ws * 4 : 0),
+                 o_gl = io.take(global ? (3 * ws + (uint64_t)ntasks * kGlobalStackInts) * 4 : 0);
+  int rc = ensure_io(h, io.total);
+  if (rc) return rc;
+  uint8_t* dev = h->io;
+  uint8_t* pin = pinned(h, std::max(in_bytes, out_bytes));
+  cudaError_t e = cudaSuccess;
+  if (pin) {
+    std::memcpy(pin + o_off, offsets, (ntasks + 1) * 8ull);
+    std::memcpy(pin + o_p, p, ntasks * 4ull);
+    if (tot) std::memcpy(pin + o_ci, cand_ids, tot * 4);
+    if (tot) std::memcpy(pin + o_cd, cand_dists, tot * 4);
+    e = cudaMemcpyAsync(dev, pin, in_bytes, cudaMemcpyHostToDevice, h->stream);
+  } else {
+    e = cudaMemcpyAsync(dev + o_off, offsets, (ntasks + 1) * 8ull, cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dev + o_p, p, ntasks * 4ull, cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess && tot) e = cudaMemcpyAsync(dev + o_ci, cand_ids, tot * 4, cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess && tot) e = cudaMemcpyAsync(dev + o_cd, cand_dists, tot * 4, cudaMemcpyHostToDevice, h->stream);
+  }
   if (e == cudaSuccess) {
     PruneArgs pa;
-    pa.ntasks = ntasks; pa.p = dp; pa.offsets = doff; pa.cand_ids = dci; pa.cand_d = dcd;
-    pa.alpha = alpha; pa.out = dout; pa.gcand = gc; pa.gkey = gk; pa.gws = gl;
-    launch_prune_tasks(view(h), pa, h->stream);
+    pa.ntasks = ntasks; pa.p = (uint32_t*)(dev + o_p); pa.offsets = (uint64_t*)(dev + o_off);
+    pa.cand_ids = (uint32_t*)(dev + o_ci); pa.cand_d = (float*)(dev + o_cd);
+    pa.alpha = alpha; pa.out = (uint32_t*)(dev + o_out);
+    pa.gcand = (uint32_t*)(dev + o_gc); pa.gkey = (float*)(dev + o_gk); pa.gws = (int*)(dev + o_gl);
+    if (global) launch_prune_tasks(view(h), pa, h->stream);
+    else launch_prune_tasks_shared(view(h), pa, most, h->stream);
     e = cudaGetLastError();
   }
-  std::vector<uint32_t> o((uint64_t)ntasks * h->Rp);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(o.data(), dout, o.size() * 4, cudaMemcpyDeviceToHost, h->stream);
+  std::vector<uint32_t> heap(pin ? 0 : (uint64_t)ntasks * h->Rp);
+  const uint32_t* o = pin ? (const uint32_t*)pin : heap.data();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync((void*)o, dev + o_out, (uint64_t)ntasks * h->Rp * 4, cudaMemcpyDeviceToHost,
+                        h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  void* fr[] = {dp, doff, dci, dcd, dout, gc, gk, gl};
-  for (void* q : fr) dfree(q);
+  else cudaStreamSynchronize(h->stream);
+  release_io(h);
   CK(e);
   for (uint32_t t = 0; t < ntasks; t++) {
     uint32_t len = 0;
@@ -1539,57 +1676,66 @@ int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   CK(cudaSetDevice(h->device));
   uint64_t rb = (uint64_t)h->d * esize(h->dtype), ds = h->stride;
   const IndexView ix = view(h);
-  // one buffer, kept with the handle up to kGtKeepBytes: allocating and freeing
-  // megabytes costs about a millisecond, more than a small call's kernels
-  constexpr uint64_t kGtKeepBytes = 1ull << 30;
-  auto r256 = [](uint64_t x) { return (x + 255) & ~(uint64_t)255; };
-  const uint64_t work_bytes = groundtruth_work_bytes(ix, nq, h->sm_count);
-  const uint64_t need = r256(nq * ds) + 2 * r256(nq * k * 4ull) + work_bytes;
-  if (need > h->gtbuf_bytes) {
-    dfree(h->gtbuf);
-    h->gtbuf = nullptr;
-    h->gtbuf_bytes = 0;
-    CK(dalloc(&h->gtbuf, need));
-    h->gtbuf_bytes = need;
-  }
-  uint8_t* dq = h->gtbuf;
-  uint32_t* di = (uint32_t*)(dq + r256(nq * ds));
-  float* dd = (float*)((uint8_t*)di + r256(nq * k * 4ull));
-  uint8_t* work = (uint8_t*)dd + r256(nq * k * 4ull);
+  IoParts io;
+  const uint64_t o_q = io.take(nq * ds), o_i = io.take(nq * k * 4ull), o_d = io.take(nq * k * 4ull),
+                 o_w = io.take(1024 + groundtruth_work_bytes(ix, nq, h->sm_count));
+  int rc = ensure_io(h, io.total);
+  if (rc) return rc;
+  uint8_t* dq = h->io + o_q;
+  uint32_t* di = (uint32_t*)(h->io + o_i);
+  float* dd = (float*)(h->io + o_d);
+  uint8_t* work = h->io + ((o_w + 1023) & ~(uint64_t)1023);
+  uint8_t* pin = pinned(h, std::max<uint64_t>(nq * ds, nq * k * 8ull + 64));
   uint8_t* parts = nullptr;
   uint32_t *over = nullptr, nover = 0;
   bool ok = true;
   cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = cudaMemsetAsync(dq, 0, nq * ds, h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpy2DAsync(dq, ds, queries, qstride, rb, nq, cudaMemcpyHostToDevice, h->stream);
+  if (pin) {
+    stage_rows(pin, ds, (const uint8_t*)queries, qstride, rb, nq);
+    e = cudaMemcpyAsync(dq, pin, nq * ds, cudaMemcpyHostToDevice, h->stream);
+  } else {
+    e = cudaMemsetAsync(dq, 0, nq * ds, h->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpy2DAsync(dq, ds, queries, qstride, rb, nq, cudaMemcpyHostToDevice, h->stream);
+  }
   if (e == cudaSuccess) {
     ok = launch_groundtruth(ix, dq, ds, nq, k, di, dd, work, h->sm_count, h->stream, &over);
     e = cudaGetLastError();
   }
   if (ok) {
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(&nover, over, 4, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    // float queries whose candidates the screen could not bound
-    const uint64_t per = (uint64_t)groundtruth_exact_chunks(ix) * k * 12;
-    const uint32_t batch = (uint32_t)std::min<uint64_t>(nover, std::max<uint64_t>(1, (256ull << 20) / per));
-    if (e == cudaSuccess && nover) e = dalloc(&parts, batch * per);
-    for (uint32_t f = 0; e == cudaSuccess && f < nover; f += batch) {
-      launch_groundtruth_exact(ix, dq, ds, nq, f, std::min(batch, nover - f), k, di, dd, work,
-                               h->sm_count, parts, h->stream);
-      e = cudaGetLastError();
+    auto download = [&]() {  // ids, distances and the word that counts what is left
+      if (pin) {
+        e = cudaMemcpyAsync(pin, di, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(pin + nq * k * 4ull, dd, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(pin + nq * k * 8ull, over, 4, cudaMemcpyDeviceToHost, h->stream);
+      } else {
+        e = cudaMemcpyAsync(ids, di, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(dists, dd, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&nover, over, 4, cudaMemcpyDeviceToHost, h->stream);
+      }
+      if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+      if (e != cudaSuccess || !pin) return;
+      std::memcpy(ids, pin, nq * k * 4ull);
+      std::memcpy(dists, pin + nq * k * 4ull, nq * k * 4ull);
+      std::memcpy(&nover, pin + nq * k * 8ull, 4);
+    };
+    if (e == cudaSuccess) download();
+    if (e == cudaSuccess && nover) {  // float queries whose candidates the screen could not bound
+      const uint32_t left = nover;
+      const uint64_t per = (uint64_t)groundtruth_exact_chunks(ix) * k * 12;
+      const uint32_t batch = (uint32_t)std::min<uint64_t>(left, std::max<uint64_t>(1, (256ull << 20) / per));
+      e = dalloc(&parts, batch * per);
+      for (uint32_t f = 0; e == cudaSuccess && f < left; f += batch) {
+        launch_groundtruth_exact(ix, dq, ds, nq, f, std::min(batch, left - f), k, di, dd, work,
+                                 h->sm_count, parts, h->stream);
+        e = cudaGetLastError();
+      }
+      if (e == cudaSuccess) download();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ids, di, nq * k * 4, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dists, dd, nq * k * 4, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   }
+  if (!ok || e != cudaSuccess) cudaStreamSynchronize(h->stream);
   dfree(parts);
-  if (h->gtbuf_bytes > kGtKeepBytes) {
-    dfree(h->gtbuf);
-    h->gtbuf = nullptr;
-    h->gtbuf_bytes = 0;
-  }
+  release_io(h);
   CK(e);
   if (!ok) return fail(h, DD_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   return check_error_word(h);

@@ -128,6 +128,51 @@ __global__ void k_prune_tasks(IndexView ix, PruneArgs pa) {
   }
 }
 
+// The same with each list in shared memory and the fast greedy forms
+// (k_prune's): lists of up to `cap` entries, out-list included.  512 tasks of
+// ~135 candidates and a full row, 100k x 100 int8: 331 us in global memory with
+// one lane per occlusion pair, 54 us here.
+template <int DT, int MT>
+__global__ void __launch_bounds__(64) k_prune_tasks_shared(IndexView ix, PruneArgs pa,
+                                                           PruneLayout lay) {
+  extern __shared__ uint4 smem_raw[];
+  const uint32_t wpc = blockDim.x >> 5, wic = threadIdx.x >> 5, lane = lane_id();
+  uint8_t* base = (uint8_t*)smem_raw + (size_t)wic * lay.total;
+  uint8_t* qv = base + lay.qv;
+  PruneSmem Pm = prune_ws((uint32_t*)(base + lay.cid), (float*)(base + lay.ckey), base + lay.ws,
+                          lay.ccap);
+  Pm.sel = (uint4*)(base + lay.ws + prune_sel_offset(lay.ccap));
+  const uint32_t qb = r16((uint64_t)ix.d * ElemSize<DT>::v);
+  for (uint32_t t = blockIdx.x * wpc + wic; t < pa.ntasks; t += gridDim.x * wpc) {
+    const uint32_t p = pa.p[t];
+    const uint64_t o0 = pa.offsets[t];
+    uint32_t m = (uint32_t)(pa.offsets[t + 1] - o0);
+    load_vec(qv, ix.points + (uint64_t)p * ix.stride, qb);
+    for (uint32_t j = lane; j < m; j += 32) {
+      Pm.cid[j] = pa.cand_ids[o0 + j];
+      Pm.ckey[j] = pa.cand_d[o0 + j];
+    }
+    __syncwarp();
+    const uint32_t* prow = ix.graph + (uint64_t)p * ix.Rp;
+    for (uint32_t b0 = 0; b0 < ix.Rp; b0 += 32) {
+      const uint32_t j = b0 + lane;
+      const uint32_t a = j < ix.Rp ? prow[j] : DD_NONE;
+      const uint32_t vb = __ballot_sync(0xffffffffu, a != DD_NONE);
+      if (a != DD_NONE) {
+        const uint32_t pos = m + __popc(vb & lanemask_lt());
+        Pm.cid[pos] = a;
+        Pm.ckey[pos] = Dist<DT, MT>::eval(qv, ix.points + (uint64_t)a * ix.stride, ix.d);
+      }
+      m += __popc(vb);
+    }
+    __syncwarp();
+    warp_std_sort(Pm, m);
+    warp_greedy_select_fast<DT, MT>(ix.points, ix.stride, ix.d, p, Pm, m, pa.alpha, ix.R,
+                                    pa.out + (uint64_t)t * ix.Rp, ix.Rp, Pm.sel);
+    __syncwarp();
+  }
+}
+
 // knn_index final step (include/index.h:133-136): per-row std::sort of the
 // neighbour ids by distance to the row's owner (ties in library order)
 template <int DT, int MT>
@@ -191,6 +236,28 @@ void launch_prune_tasks(const IndexView& ix, const PruneArgs& pa, cudaStream_t s
   if (!pa.ntasks) return;
   int grid = (int)std::min<uint32_t>(pa.ntasks, 4096);
 #define CALL(DT, MT) k_prune_tasks<DT, MT><<<grid, 32, 0, st>>>(ix, pa);
+  DD_DISPATCH_DM(ix.dtype, ix.metric, CALL);
+#undef CALL
+}
+
+static PruneLayout prune_tasks_layout(const IndexView& ix, uint64_t most) {
+  return make_prune_layout(ix.d, ix.dtype, ix.Rp, (uint32_t)most + ix.Rp, true);
+}
+
+bool prune_tasks_in_shared(const IndexView& ix, uint64_t most) {
+  // two warps a CTA
+  return most <= 4096 && 2ull * prune_tasks_layout(ix, most).total <= 227 * 1024;
+}
+
+void launch_prune_tasks_shared(const IndexView& ix, const PruneArgs& pa, uint64_t most,
+                               cudaStream_t st) {
+  if (!pa.ntasks) return;
+  const PruneLayout lay = prune_tasks_layout(ix, most);
+  const size_t sm = 2ull * lay.total;
+  const int grid = (int)std::min<uint32_t>((pa.ntasks + 1) / 2, 4096);
+#define CALL(DT, MT)                                                                 \
+  set_smem(k_prune_tasks_shared<DT, MT>, sm);                                        \
+  k_prune_tasks_shared<DT, MT><<<grid, 64, sm, st>>>(ix, pa, lay);
   DD_DISPATCH_DM(ix.dtype, ix.metric, CALL);
 #undef CALL
 }

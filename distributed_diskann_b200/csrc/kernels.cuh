@@ -247,6 +247,11 @@ struct PruneArgs {
   uint32_t* gcand; float* gkey; int* gws;
 };
 void launch_prune_tasks(const IndexView& ix, const PruneArgs& pa, cudaStream_t st);
+// the same with the lists in shared memory, when the longest one (`most`
+// candidates) fits; gcand, gkey and gws are not used
+bool prune_tasks_in_shared(const IndexView& ix, uint64_t most);
+void launch_prune_tasks_shared(const IndexView& ix, const PruneArgs& pa, uint64_t most,
+                               cudaStream_t st);
 
 // brute-force ground truth (k_gt.cu): device queries of stride qstride (a
 // multiple of 64, zero padded), a workspace of groundtruth_work_bytes; *over
