@@ -1678,7 +1678,7 @@ int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   const IndexView ix = view(h);
   IoParts io;
   const uint64_t o_q = io.take(nq * ds), o_i = io.take(nq * k * 4ull), o_d = io.take(nq * k * 4ull),
-                 o_w = io.take(1024 + groundtruth_work_bytes(ix, nq, h->sm_count));
+                 o_w = io.take(1024 + groundtruth_work_bytes(ix, nq, k, h->sm_count));
   int rc = ensure_io(h, io.total);
   if (rc) return rc;
   uint8_t* dq = h->io + o_q;

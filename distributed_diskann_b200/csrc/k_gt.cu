@@ -171,7 +171,7 @@ struct GtShape {
   uint32_t smem;
   uint32_t dp;        // float: elements of a converted row
   uint64_t slab, nslabs, qtiles, btiles, grid, per, segs;  // of a slab
-  uint64_t gtiles;    // base tiles of a sample group (0: no sample)
+  uint64_t groups, gtiles;  // sample groups (0: no sample) and their base tiles
 };
 // The first thresholds: the scores of kGtGroups groups of sampled base tiles
 // are reduced to each group's largest, and the k-th largest of those is a
@@ -180,10 +180,11 @@ struct GtShape {
 // sample's threshold a fraction of that, and lists are dearer than products:
 // without a sample 14.7 ms (10,000 x 1M x 128 uint8) and 6.6 ms (1000 x 400k x
 // 200 float), with 1/16 of the base 6.6 / 1.1, 1/8 5.4 / 0.9, 1/4 4.6 / 1.0.
-// Below 1024 tiles the sample's two launches cost more than they save.
+// A base of few tiles is sampled whole, a group a tile (99 x 67,546 x 87 uint8
+// 1.48 ms without the sample); one of fewer than k tiles is not.
 constexpr uint32_t kGtGroups = 128, kGtSampleOf = 5;
 
-static GtShape gt_shape(const IndexView& ix, uint64_t nq, int sm_count) {
+static GtShape gt_shape(const IndexView& ix, uint64_t nq, uint32_t k, int sm_count) {
   GtShape s{};
   s.f32 = ix.dtype == DD_F32;
   s.dp = (ix.d + 15) & ~15u;
@@ -206,7 +207,8 @@ static GtShape gt_shape(const IndexView& ix, uint64_t nq, int sm_count) {
   s.grid = std::min<uint64_t>(sm_count, total);
   s.per = (total + s.grid - 1) / s.grid;
   s.segs = (s.btiles - 1) / s.per + 2;
-  s.gtiles = s.btiles >= 1024 ? std::max<uint64_t>(1, s.btiles / (kGtSampleOf * kGtGroups)) : 0;
+  s.groups = s.btiles >= k ? std::min<uint64_t>(kGtGroups, s.btiles) : 0;
+  s.gtiles = std::max<uint64_t>(1, s.btiles / (kGtSampleOf * kGtGroups));
   return s;
 }
 
@@ -229,7 +231,7 @@ static GtWork gt_work(const IndexView& ix, uint64_t nq, const GtShape& s) {
   w.scal = take(64);  // [0] largest |p|^2 bits, [1] overflowed queries
   w.over = take(4 * nq);
   w.cnt = take(4 * lists);
-  w.gmax = take(s.gtiles ? 4ull * nq * kGtGroups : 0);
+  w.gmax = take(s.groups ? 4ull * nq * kGtGroups : 0);
   w.zero1 = off;
   w.thr0 = take(4 * nq);
   w.over_list = take(4 * nq);
@@ -245,8 +247,8 @@ static GtWork gt_work(const IndexView& ix, uint64_t nq, const GtShape& s) {
   return w;
 }
 
-uint64_t groundtruth_work_bytes(const IndexView& ix, uint64_t nq, int sm_count) {
-  return gt_work(ix, nq, gt_shape(ix, nq, sm_count)).total;
+uint64_t groundtruth_work_bytes(const IndexView& ix, uint64_t nq, uint32_t k, int sm_count) {
+  return gt_work(ix, nq, gt_shape(ix, nq, k, sm_count)).total;
 }
 
 // ============================================================ preparation
@@ -967,10 +969,10 @@ static bool gt_tensor_map(CUtensorMap* m, bool f32, const void* p, uint64_t row_
 template <bool F32, int MT, int MTILES>
 static void gt_launch(const GtShape& s, const CUtensorMap& qm, const CUtensorMap& bm, GtArgs g,
                       uint32_t* thr0, int sm_count, cudaStream_t st) {
-  if (s.gtiles && g.id0 == 0) {  // the first slab's sample serves all slabs
+  if (s.groups && g.id0 == 0) {  // the first slab's sample serves all slabs
     GtArgs a = g;
     a.gtiles = (uint32_t)s.gtiles;
-    a.btiles = (uint32_t)(kGtGroups * s.gtiles);
+    a.btiles = (uint32_t)(s.groups * s.gtiles);
     a.gstride = (uint32_t)(s.btiles / a.btiles);
     const uint64_t total = s.qtiles * a.btiles, grid = std::min<uint64_t>(sm_count, total);
     a.per = (uint32_t)((total + grid - 1) / grid);
@@ -979,7 +981,7 @@ static void gt_launch(const GtShape& s, const CUtensorMap& qm, const CUtensorMap
     k_gt_first<F32, MT><<<(unsigned)((g.nq + 7) / 8), 256, 0, st>>>(g.gmax, g.nq, g.k, g.qnorm,
                                                                     g.pmax, g.d, thr0);
   }
-  g.thr0 = s.gtiles ? thr0 : nullptr;
+  g.thr0 = s.groups ? thr0 : nullptr;
   set_smem(k_gt_tc<F32, MT, MTILES, false>, s.smem);
   k_gt_tc<F32, MT, MTILES, false><<<(unsigned)s.grid, MTILES * 128 + 64, s.smem, st>>>(qm, bm, g);
 }
@@ -990,7 +992,7 @@ static void gt_launch(const GtShape& s, const CUtensorMap& qm, const CUtensorMap
 bool launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qstride, uint64_t nq,
                         uint32_t k, uint32_t* ids, float* dists, uint8_t* work, int sm_count,
                         cudaStream_t st, uint32_t** over) {
-  const GtShape s = gt_shape(ix, nq, sm_count);
+  const GtShape s = gt_shape(ix, nq, k, sm_count);
   const GtWork w = gt_work(ix, nq, s);
   const bool l2 = ix.metric == DD_L2;
   cudaMemsetAsync(work + w.zero0, 0, w.zero1 - w.zero0, st);
@@ -1098,7 +1100,7 @@ void launch_groundtruth_exact(const IndexView& ix, const uint8_t* queries, uint6
                               uint64_t nq, uint32_t first, uint32_t count, uint32_t k,
                               uint32_t* ids, float* dists, const uint8_t* work, int sm_count,
                               uint8_t* parts, cudaStream_t st) {
-  const GtWork w = gt_work(ix, nq, gt_shape(ix, nq, sm_count));
+  const GtWork w = gt_work(ix, nq, gt_shape(ix, nq, k, sm_count));
   const uint32_t* list = (const uint32_t*)(work + w.over_list) + first;
   const uint32_t nchunks = groundtruth_exact_chunks(ix);
   double* pd = (double*)parts;
