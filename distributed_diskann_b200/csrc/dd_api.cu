@@ -1374,6 +1374,7 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   qa.cls_items = nullptr;
   qa.cls_count = nullptr;
   qa.cls_queue = nullptr;
+  qa.repeats = nullptr;
   qa.Lvalid = Lmax;
   qa.hash_scratch = nullptr;
   // Evicted lists (visited entries pushed out of the frontier, which a query
@@ -1411,7 +1412,7 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   // each class runs as a persistent launch laid out for its own beam width
   // (smaller hash table and frontier: more resident queries per SM), largest
   // class first; classes without queries end at once
-  const uint64_t words = (uint64_t)kQueryClasses * nq + 2 * kQueryClasses;
+  const uint64_t words = (uint64_t)kQueryClasses * nq + 2 * kQueryClasses + 1;
   if (words > h->qcls_words) {
     dfree(h->qcls);
     h->qcls = nullptr;
@@ -1421,6 +1422,7 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   }
   uint32_t* counts = h->qcls + (uint64_t)kQueryClasses * nq;
   uint32_t* queues = counts + kQueryClasses;
+  qa.repeats = queues + kQueryClasses;
   IndexView ixq = view(h);
   if (screen_enabled(h)) {  // float data: BF16 screen, exact re-rank
     int rc = ensure_screen(h);
@@ -1428,7 +1430,7 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
     attach_screen(h, &ixq);
   }
   ixq.fgroup_lg = fast_fgroup(h);
-  CK(cudaMemsetAsync(counts, 0, 2 * kQueryClasses * 4, h->stream));
+  CK(cudaMemsetAsync(counts, 0, (2 * kQueryClasses + 1) * 4, h->stream));
   // one class: every query is its, no list needed
   const bool one = (classes & (classes - 1)) == 0;
   h->launches = 0;
@@ -1444,7 +1446,7 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
     // queries per SM by shared memory: they go to one global slice per warp
     const bool hglob = hash_table_bytes(hash_bits_for(Lc), use_h24(h)) > 16384;
     WarpLayout lc = make_search_layout(h->d, h->dtype, h->metric, Lc, h->Rp, 2 * Lc + 64, false,
-                                       use_h24(h), false, false, hglob);
+                                       use_h24(h), false, true, hglob);
     const LaunchPlan plan = query_plan(h, lc, Lc);
     QueryArgs qc = qa;
     qc.Lmax = Lc;

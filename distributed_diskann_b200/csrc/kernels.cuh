@@ -24,7 +24,7 @@ struct WarpLayout {
   uint32_t hash_words;   // its size in 32-bit words (16-byte multiple)
   uint32_t ev;           // query layout: evicted list in shared memory (keep_vis layouts)
   uint32_t term;         // float L2: sums of the distances in progress
-  uint32_t nf;           // fast build search: padded frontier of 64-bit keys (0: id / distance arrays)
+  uint32_t nf;           // fast searches: padded frontier of 64-bit keys (0: id / distance arrays)
 };
 
 // Per-warp shared-memory carve-up of k_prune (byte offsets, 16-byte aligned).
@@ -63,7 +63,8 @@ struct IndexView {
 
 // keep_vis: the query layout reserves the visited list (k_beam keeps it;
 // k_query only needs the evicted list)
-// fastf (build only): the fast form's seen filter, 16-bit tags (search_core.cuh)
+// fastf: the fast form's build search (seen filter of 16-bit tags) or query
+// search (64-bit frontier keys, beam widths up to 256) (search_core.cuh)
 // hash_global (query only): the seen table goes to a global slice per resident
 // warp (QueryArgs::hash_scratch) instead of shared memory
 WarpLayout make_search_layout(uint32_t d, int dtype, int metric, uint32_t L, uint32_t Rp, uint32_t vcap,
@@ -191,6 +192,7 @@ struct QueryArgs {
   const uint32_t* cls_items;
   const uint32_t* cls_count;
   uint32_t* cls_queue;
+  uint32_t* repeats;       // fast form: set once a search met a candidate twice in a step
   uint32_t Lvalid;         // largest valid beam width (the caller's Lmax; Lmax is the class's)
   uint32_t* hash_scratch;  // layouts with hash_global: one table per warp of the grid
   uint32_t* ev_scratch;    // evicted lists, ev_cap ids per warp of the grid

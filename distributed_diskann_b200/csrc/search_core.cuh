@@ -1483,4 +1483,278 @@ __device__ SearchOut warp_build_search(const SearchParams& P, const SearchSmem& 
   return o;
 }
 
+// ---------------------------------------------------------------------------
+// The query search of the fast form (beam widths up to 32 FPL): the results of
+// warp_beam_search in query mode, with warp_build_search's frontier.  What a
+// query adds: the reference's lossy filter replayed exactly, the limits on
+// visits and degree, the k-cut and the evicted list.  It is made for searches
+// whose steps never hold a candidate twice, which rows without repeated ids
+// guarantee; a step that does (two of its candidates fall on one slot of the
+// merged frontier) ends the search and returns false: the frontier is then a
+// multiset, and the caller runs warp_beam_search instead.
+//
+// A query is bound by the latency of its steps (15 searches share an SM at L =
+// 100, where the reference's 12 KB filter tables fill the shared memory), so
+// what counts here is the length of the chain from a row to the next one.
+// Measured on B200, k_query against warp_beam_search's: one query of 100k x 64
+// f32 at L = 100 361 -> 301 us, 10,000 at L = 50 1.39 -> 1.22 ms, 10,000 of 100k
+// x 100 int8 at L = 200 5.16 -> 4.70 ms, 50,000 inner-product queries of 400k x
+// 200 f32 at L = 50 10.9 -> 10.6 ms, 10,000 of 1M x 128 uint8 at L = 100 2.41 ->
+// 2.36 ms; at L = 10 (14 steps, mostly fetching code) 71.7 -> 73 us.
+// ---------------------------------------------------------------------------
+template <int DT, int MT, int FPL, int CPL>
+__device__ bool warp_query_search(const SearchParams& P, const SearchSmem& S, uint32_t self_id,
+                                  SearchOut* out) {
+  constexpr uint32_t NF = 32 * FPL;
+  constexpr uint32_t FULL = 0xffffffffu;
+  typedef unsigned long long u64;
+  const uint32_t lane = lane_id(), lt = lanemask_lt(), gt = lanemask_gt();
+  u64* const fr = (u64*)S.fr_id;
+  u64* const cand = (u64*)S.c_id;
+  const uint32_t nslots = 1u << P.hbits, hmask = nslots - 1;
+  const uint32_t n32 = (uint32_t)P.n, row_bytes = P.Rp * 4u;
+  auto key_of = [](uint32_t id, float d) {
+    return ((u64)dist_order<MT>(d) << 32) | (id << 1);
+  };
+  auto lo32 = [](u64 k) { return (uint32_t)k; };
+  auto hi32 = [](u64 k) { return (uint32_t)(k >> 32); };
+  {
+    uint4* h4 = (uint4*)S.hash;
+    const uint4 none = make_uint4(DD_NONE, DD_NONE, DD_NONE, DD_NONE);
+    const uint32_t n16 = hash_table_bytes(P.hbits, S.h24 != 0) / 16u;
+    for (uint32_t i = lane; i < n16; i += 32) h4[i] = none;
+    S.ev_bloom[lane] = 0u;
+#pragma unroll
+    for (int t = 0; t < FPL; t++) fr[32 * t + lane] = ~0ull;
+  }
+  const float d_start = point_dist<DT, MT>(P, S.qv, P.start);
+  u64 cur = key_of(P.start, d_start);
+  if (d_start != d_start) cur = ((u64)0xfffffffeu << 32) | (P.start << 1);  // NaN: last
+  __syncwarp();
+  if (lane == 0) fr[0] = cur;
+  uint32_t U[FPL];  // unvisited positions
+#pragma unroll
+  for (int t = 0; t < FPL; t++) U[t] = t == 0 ? 1u : 0u;
+  auto first_unvisited = [&]() {
+    int p = -1;
+#pragma unroll
+    for (int t = FPL - 1; t >= 0; t--)
+      if (U[t]) p = 32 * t + __ffs(U[t]) - 1;
+    return p;
+  };
+  uint32_t ev_n = 0;
+  // the visited ones of this lane's evicted entry, in lane order
+  auto evict = [&](u64 o) {
+    const bool v = (o & 1ull) != 0ull;
+    const uint32_t vb = __ballot_sync(FULL, v);
+    if (v) {
+      const uint32_t pos = ev_n + __popc(vb & lt), id = lo32(o) >> 1;
+      if (pos < P.ecap) {
+        S.ev_id[pos] = id;
+        ev_bloom_add(S.ev_bloom, id);
+      } else {
+        dd_set_error(P.err, DD_EVIS_CAP);
+      }
+    }
+    ev_n = min(P.ecap, ev_n + __popc(vb));
+  };
+  uint32_t fr_n = 1, cmps = 1, visits = 0;
+  const float int_max_f = 2147483648.0f;  // (float)std::numeric_limits<int>::max()
+  const uint32_t dl = min(P.degree_limit, P.Rp);
+  const uint32_t limit = (uint32_t)min(P.limit, (uint64_t)0xffffffffu);
+  uint32_t a_pre[CPL], pre = DD_NONE;
+  auto prefetch_row = [&](uint32_t node) {
+    pre = node;
+    const uint32_t* prow = (const uint32_t*)((const uint8_t*)P.graph + (uint64_t)node * row_bytes);
+#pragma unroll
+    for (int t = 0; t < CPL; t++) {
+      const uint32_t j = 32 * t + lane;
+      a_pre[t] = (j < dl) ? __ldg(prow + j) : DD_NONE;
+    }
+  };
+  prefetch_row(P.start);
+  uint32_t cur_pos = 0;
+  __syncwarp();
+  while (visits < limit) {
+    // ---- visit `cur` (at cur_pos, its row in a_pre)
+    const float cutoff = fr_n >= P.L ? order_dist<MT>(hi32(fr[fr_n - 1])) : int_max_f;
+    if (lane == 0) ((uint32_t*)(fr + cur_pos))[0] = lo32(cur) | 1u;
+#pragma unroll
+    for (int t = 0; t < FPL; t++)
+      if ((cur_pos >> 5) == (uint32_t)t) U[t] &= ~(1u << (cur_pos & 31));
+    visits++;
+    const int nxt_pos = first_unvisited();
+    u64 nxt = ~0ull;
+    if (nxt_pos >= 0) {
+      nxt = fr[nxt_pos];
+      if (lane * 32u < dl) {  // its row to L2 (128-byte lines, one per lane)
+        const uint8_t* nrow =
+            (const uint8_t*)P.graph + (uint64_t)(lo32(nxt) >> 1) * row_bytes + lane * 128u;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(nrow));
+      }
+    }
+    // ---- the lossy filter, replayed chunk by chunk in neighbour order
+    uint32_t loc[CPL], grp[CPL], prev_a[CPL];
+    bool part[CPL];
+#pragma unroll
+    for (int t = 0; t < CPL; t++) {
+      const uint32_t at = a_pre[t];
+      if (at >= n32 && at != DD_NONE) dd_set_error(P.err, DD_EBAD_ID);
+      part[t] = at < n32 && at != self_id;
+      loc[t] = part[t] ? (uint32_t)(dd_hash64(at) & hmask) : (0x80000000u | lane);
+    }
+#pragma unroll
+    for (int t = 0; t < CPL; t++) {
+      grp[t] = __match_any_sync(FULL, loc[t]);
+      const uint32_t before = grp[t] & lt;
+      prev_a[t] = __shfl_sync(FULL, a_pre[t], before ? 31 - __clz(before) : lane);
+    }
+    uint32_t nk = 0;
+#pragma unroll
+    for (int t = 0; t < CPL; t++) {
+      const uint32_t before = grp[t] & lt;
+      const uint32_t tval = (part[t] && !before) ? hash_get(S, nslots, loc[t]) : DD_NONE;
+      const bool keep = part[t] && (before ? prev_a[t] : tval) != a_pre[t];
+      const uint32_t kb = __ballot_sync(FULL, keep);
+      if (part[t] && (grp[t] & gt) == 0) hash_set(S, nslots, loc[t], a_pre[t]);
+      if (keep) S.s_id[nk + __popc(kb & lt)] = a_pre[t];
+      nk += __popc(kb);
+      __syncwarp();
+    }
+    cmps += nk;
+    // ---- distances; those below the cutoff become keys
+    const uint32_t nc = step_distances<DT, MT, 8, false>(
+        P, S, nk, cutoff, cutoff < int_max_f,
+        [&](uint32_t pos, uint32_t id, float dist) { cand[pos] = key_of(id, dist); });
+    __syncwarp();
+    if (nc == 0 && nxt_pos >= 0) prefetch_row(lo32(nxt) >> 1);
+    u64 next = nxt;
+    bool grew = false;
+    for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
+      u64 c = c0 + lane < nc ? cand[c0 + lane] : ~0ull;
+      for (uint32_t e = 0; e < c0; e++)  // (more than 32 candidates) a copy in an earlier group
+        if (__any_sync(FULL, cand[e] == c)) return false;
+      uint32_t lo = 0;
+#pragma unroll
+      for (uint32_t step = NF / 2; step; step >>= 1)
+        if (fr[lo + step - 1] < c) lo += step;
+      const u64 at = fr[lo];
+      const bool keep = c != ~0ull && (at >> 1) != (c >> 1);
+      const uint32_t K = __ballot_sync(FULL, keep);
+      const bool last_group = c0 + 32 >= nc;
+      // of two copies of an entry that the frontier holds, the second is kept
+      const bool held = c != ~0ull && !keep;
+      if (__popc(__ballot_sync(FULL, held)) > 1) {
+        const uint32_t same = __match_any_sync(FULL, held ? lo32(c) : (lane << 1) | 1u);
+        if (__any_sync(FULL, held && __popc(same) > 1)) return false;
+      }
+      if (!K) {
+        if (last_group && next != ~0ull) prefetch_row(lo32(next) >> 1);
+        continue;
+      }
+      grew = true;
+      const uint32_t nkeep = __popc(K);
+      uint32_t rank = 0;
+      for (uint32_t km = K; km; km &= km - 1)
+        rank += __shfl_sync(FULL, c, __ffs(km) - 1) < c ? 1u : 0u;
+      const uint32_t dst = keep ? lo + rank : NF;
+      uint32_t M[FPL], slots = 0;  // candidate slots
+#pragma unroll
+      for (int t = 0; t < FPL; t++) {
+        M[t] = __reduce_or_sync(FULL, (dst >> 5) == (uint32_t)t ? 1u << (dst & 31) : 0u);
+        slots += __popc(M[t]);
+      }
+      // equal candidates share a slot (one beyond the array: look at them all)
+      const uint32_t in_array = __popc(__ballot_sync(FULL, keep && dst < NF));
+      bool twice = slots != in_array;
+      if (in_array != nkeep) {
+        uint32_t same = 0;
+        for (uint32_t km = K; km; km &= km - 1)
+          same += __shfl_sync(FULL, c, __ffs(km) - 1) == c ? 1u : 0u;
+        twice = __any_sync(FULL, keep && same > 1);
+      }
+      if (twice) return false;
+      // a candidate that was visited and pushed out before comes back visited
+      bool again = false;
+      if (ev_n && keep && ev_bloom_maybe(S.ev_bloom, lo32(c) >> 1))
+        for (uint32_t e = 0; e < ev_n; e++) again |= S.ev_id[e] == lo32(c) >> 1;
+      const uint32_t ab = __ballot_sync(FULL, again);
+      {
+        const uint32_t fb = __ballot_sync(FULL, keep && rank == 0);
+        const u64 best = __shfl_sync(FULL, c, __ffs(fb) - 1);
+        if (!(fb & ab) && best < next) next = best;
+      }
+      if (last_group && next != ~0ull) prefetch_row(lo32(next) >> 1);
+      if (again) c |= 1ull;
+      const uint32_t total = fr_n + nkeep, new_n = min(P.L, total);
+      if (total > new_n) {  // visited entries pushed off the end are remembered
+        const uint32_t off = total - new_n - __popc(__ballot_sync(FULL, keep && dst >= new_n));
+        if (off) evict(lane < off ? fr[fr_n - off + lane] : 0ull);
+      }
+      __syncwarp();
+      uint32_t upto = slots;
+#pragma unroll
+      for (int t = FPL - 1; t >= 0; t--) {
+        if (upto) {
+          const uint32_t below = upto - __popc(M[t]);
+          const uint32_t s = 32 * t + lane;
+          const bool in = s < new_n, isc = (M[t] >> lane) & 1u;
+          const u64 v = in ? fr[s - below - __popc(M[t] & lt)] : ~0ull;
+          __syncwarp();
+          if (in && !isc) fr[s] = v;
+          U[t] = __ballot_sync(FULL, in && (isc || !(v & 1ull)));
+          upto = below;
+        }
+      }
+      if (dst < new_n) fr[dst] = c;
+      for (uint32_t b = ab; b; b &= b - 1) {
+        const uint32_t d = __shfl_sync(FULL, dst, __ffs(b) - 1);
+#pragma unroll
+        for (int t = 0; t < FPL; t++)
+          if ((d >> 5) == (uint32_t)t) U[t] &= ~(1u << (d & 31));
+      }
+      fr_n = new_n;
+      __syncwarp();
+    }
+    // ---- k-cut (metric spaces only): entries up to cut * dist(k) stay
+    if (grew && MT == DD_L2 && P.k > 0 && fr_n > P.k) {
+      const float thr = (float)(P.cut * (double)order_dist<MT>(hi32(fr[P.k])));
+      if (!(order_dist<MT>(hi32(fr[fr_n - 1])) < thr)) {
+        uint32_t keep_n = 0;
+#pragma unroll
+        for (int t = 0; t < FPL; t++) {
+          const uint32_t s = 32 * t + lane;
+          const u64 o = fr[s];
+          const float fd = order_dist<MT>(hi32(o));
+          keep_n += __popc(__ballot_sync(
+              FULL, s < fr_n && ((fd < thr) || (fd == thr && (lo32(o) >> 1) == 0))));
+        }
+#pragma unroll
+        for (int t = 0; t < FPL; t++) {
+          const uint32_t s = 32 * t + lane;
+          if (32u * t < fr_n && 32u * t + 32 > keep_n) {
+            const bool drop = s >= keep_n && s < fr_n;
+            evict(drop ? fr[s] : 0ull);
+            if (drop) fr[s] = ~0ull;
+            const uint32_t kept = keep_n > 32u * t ? (1u << (keep_n - 32 * t)) - 1u : 0u;
+            U[t] &= kept;
+          }
+        }
+        fr_n = keep_n;
+        __syncwarp();
+      }
+    }
+    // ---- the next node
+    const int np = first_unvisited();
+    if (np < 0) break;
+    cur_pos = (uint32_t)np;
+    cur = fr[cur_pos];
+    if (pre != lo32(cur) >> 1) prefetch_row(lo32(cur) >> 1);
+  }
+  out->fr_n = fr_n;
+  out->vis_n = visits;
+  out->cmps = cmps;
+  return true;
+}
+
 }  // namespace ddk
