@@ -652,10 +652,9 @@ int pass_rounds(dd_index* h, const std::vector<std::pair<uint64_t, uint64_t>>& r
     ReverseScratch rs = make_rs(h, res);
     rs.split = bp.fast && B * h->Rp >= kRevSplitPairs;
     launch_reverse(ix, ra, rs, bp.fast, h->stream, h->sm_count, h->fork);
-    // k_search, k_prune, k_apply_rows, k_reverse, k_reverse_big, and k_rev_split,
-    // k_rev_short of split rounds; per radix pass a histogram, three scans and
-    // a scatter; the segment heads' flags, three scans and scatter
-    h->launches += 10 + (rs.split ? 2 : 0) + 5 * (uint64_t)((64 - __builtin_clzll(h->n > 1 ? h->n - 1 : 1) + 7) / 8);
+    // k_search, k_prune, k_apply_rows, k_reverse, k_reverse_big, the sort's, and
+    // k_rev_split, k_rev_short of split rounds
+    h->launches += 5 + ss.launches + (rs.split ? 2 : 0);
     if (P->collect_stats) {
       k_accumulate<<<64, 256, 0, h->stream>>>(h->stat_vis, h->stat_cmps, (uint32_t)B, h->counters,
                                               h->acc);

@@ -25,6 +25,7 @@ struct SemisortScratch {
   // owner filter of a sharded build: only targets t with t % world == rank
   // are kept (world = 1: every target)
   uint32_t world = 1, rank = 0;
+  uint32_t launches = 0;  // kernels launched
 };
 
 // Sorts the valid entries of new_out (E = B*Rp, DD_NONE = empty slot) by
