@@ -1669,12 +1669,9 @@ int dd_robust_prune(dd_index* h, uint32_t ntasks, const uint32_t* p, const uint6
   return check_error_word(h);
 }
 
-int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride, uint32_t k,
-                   uint32_t* ids, float* dists) {
-  if (!h || !queries || !ids || !dists) return DD_ERR_ARG;
-  if (k == 0 || k > 32 || k > h->n) return fail(h, DD_ERR_UNSUPPORTED, "k must be in [1, 32]");
-  if (nq == 0) return DD_OK;
-  CK(cudaSetDevice(h->device));
+// one launch of the ground truth: nq queries, arguments checked
+static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
+                             uint32_t k, uint32_t* ids, float* dists) {
   uint64_t rb = (uint64_t)h->d * esize(h->dtype), ds = h->stride;
   const IndexView ix = view(h);
   IoParts io;
@@ -1740,6 +1737,26 @@ int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   CK(e);
   if (!ok) return fail(h, DD_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   return check_error_word(h);
+}
+
+int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride, uint32_t k,
+                   uint32_t* ids, float* dists) {
+  if (!h || !queries || !ids || !dists) return DD_ERR_ARG;
+  if (k == 0 || k > 32 || k > h->n) return fail(h, DD_ERR_UNSUPPORTED, "k must be in [1, 32]");
+  if (nq == 0) return DD_OK;
+  CK(cudaSetDevice(h->device));
+  // the lists take 1 KB a query and segment: as many queries at a time as keep the
+  // workspace within 2 GB, but at least 4096 (a float base is converted once a batch)
+  const IndexView ix = view(h);
+  uint64_t batch = nq;
+  while (batch > 4096 && groundtruth_work_bytes(ix, batch, k, h->sm_count) > (2ull << 30))
+    batch = (batch + 1) / 2;
+  for (uint64_t q = 0; q < nq; q += batch) {
+    const int rc = groundtruth_batch(h, (const uint8_t*)queries + q * qstride, std::min(batch, nq - q),
+                                     qstride, k, ids + q * k, dists + q * k);
+    if (rc) return rc;
+  }
+  return DD_OK;
 }
 
 // the caller may write the points through this pointer: the BF16 row copies

@@ -16,8 +16,8 @@
 // tiles of 128 points; one thread issues the tcgen05.mma of a tile while the
 // epilogue warps read the other TMEM buffer: thread r of a query tile owns
 // query r (TMEM lane r), keeps its threshold in a register and appends the few
-// values that pass to the query's list.  The (query tile, base tile) steps are
-// split evenly over one CTA per SM.
+// values that pass to the query's list in global memory.  The (query tile, base
+// tile) steps are split evenly over one CTA per SM.
 //
 // Integer data: one score per pair, 2 q.p - |p|^2 (L2) or q.p (MIPS), exact in
 // 32 bits; the list keeps the k best.  Float data: rows are split x = hi + lo
@@ -29,8 +29,8 @@
 // against every point.
 //
 // Measured on B200, all kernels of a call: 10,000 x 1M x 128 uint8, k = 32: 144
-// ms (mma.sync tiles of 16 queries a warp) -> 4.9 ms; 1000 x 400k x 200 float
-// inner product: 185 ms (FP64 on the CUDA cores, one row per lane) -> 1.3 ms.
+// ms (mma.sync tiles of 16 queries a warp) -> 4.4 ms; 1000 x 400k x 200 float
+// inner product: 185 ms (FP64 on the CUDA cores, one row per lane) -> 1.2 ms.
 // What bounds it now: the epilogue (two instructions a value, and the lists),
 // not the products (0.6 ms of the uint8 call at the measured GEMM rate).
 #include <cfloat>
@@ -151,10 +151,13 @@ __global__ void k_gt_merge_parts(const double* part_d, const uint32_t* part_i, c
 constexpr uint32_t kGtTile = 128;      // base points of a tile (accumulator columns)
 constexpr uint32_t kGtBlockBytes = 128;             // bytes of a row in one k-block
 constexpr uint32_t kGtTileBytes = kGtTile * kGtBlockBytes;
-// entries of a query's list in shared memory, and the most a compaction leaves
-// (8 may come before the next one)
-__host__ __device__ constexpr uint32_t gt_cap(bool f32) { return f32 ? 47 : 48; }
-constexpr uint32_t kGtKeep = 40;
+// entries of a query's list of one segment; a compaction leaves at most 8 fewer.
+// The lists are in global memory (L2): appends are stores that nothing waits
+// for, and with the sample's thresholds about 50 values come to a list, so that
+// it is hardly ever compacted.  (In shared memory a list held 48: some warp
+// compacted one in most steps, and the step's TMEM buffer waited for it: 4.3 ms
+// instead of 3.7 ms for the uint8 call below.)
+constexpr uint32_t kGtCap = 128;
 constexpr uint64_t kGtSlab = 1u << 20; // float base rows converted at a time
 // |p|^2 of the rows past n, and the scores that no point lies below and no such
 // row reaches (integer rows of 1024 bytes: scores above -2^27)
@@ -195,8 +198,8 @@ static GtShape gt_shape(const IndexView& ix, uint64_t nq, uint32_t k, int sm_cou
   // epilogue of 128 queries would ask more of L2 than it gives)
   s.mtiles = (!s.f32 && s.nkb == 1) ? 2 : 1;
   s.rows = 128 * s.mtiles;
-  // queries | lists | the epilogue warps' norms; 1 KB is static (barriers)
-  const uint32_t fixed = s.mtiles * s.nkb * kGtTileBytes + s.rows * gt_cap(s.f32) * 8 + s.rows * 16;
+  // queries | the epilogue warps' norms; 1 KB is static (barriers)
+  const uint32_t fixed = s.mtiles * s.nkb * kGtTileBytes + s.rows * 16;
   s.stages = std::min<uint32_t>(8, (226 * 1024 - fixed) / kGtTileBytes);
   s.smem = fixed + s.stages * kGtTileBytes;
   s.slab = s.f32 ? std::min<uint64_t>(ix.n, kGtSlab) : ix.n;
@@ -237,8 +240,8 @@ static GtWork gt_work(const IndexView& ix, uint64_t nq, const GtShape& s) {
   w.over_list = take(4 * nq);
   w.qnorm = take(4 * nq);
   w.pnorm = take(4 * s.btiles * kGtTile);
-  w.ent_v = take(4 * lists * kGtKeep);
-  w.ent_i = take(4 * lists * kGtKeep);
+  w.ent_v = take(4 * lists * kGtCap);
+  w.ent_i = take(4 * lists * kGtCap);
   if (s.f32) {
     w.bhalf = take(2ull * s.slab * 2 * s.dp);
     w.qhalf = take(2ull * nq * 2 * s.dp);
@@ -422,7 +425,7 @@ struct GtArgs {
   const uint32_t* pmax;    // float data: bits of the largest |p|^2
   uint32_t* over;          // float data: queries the screen gave up
   uint32_t* cnt;
-  uint32_t* ent_v;         // [list tile][kGtKeep][rows]
+  uint32_t* ent_v;         // [list tile][kGtCap][rows]
   uint32_t* ent_i;
   uint32_t* err;
   // sample launch: tile i of the sample is base tile i * gstride, its group i / gtiles
@@ -460,7 +463,6 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
             GtArgs g) {
   constexpr uint32_t ROWS = 128 * MTILES;
   constexpr uint32_t EW = 4 * MTILES;  // epilogue warps; then the producer, then the issuer
-  constexpr uint32_t CAP = gt_cap(F32);
   constexpr int KB = F32 ? 64 : 128;  // elements of a k-block
   constexpr uint32_t FULL = 0xffffffffu;
   extern __shared__ __align__(1024) uint8_t smem_gt[];
@@ -476,9 +478,7 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
   const uint32_t qs = smem_u32(base);                                   // query blocks
   const uint32_t bs = qs + MTILES * g.nkb * kGtTileBytes;               // base stages
   uint8_t* after = base + (MTILES * g.nkb + g.stages) * kGtTileBytes;
-  uint32_t* lv = (uint32_t*)after;           // [CAP][ROWS] scores
-  uint32_t* li = lv + CAP * ROWS;            // [CAP][ROWS] ids
-  uint32_t* pn_s = li + CAP * ROWS;          // [EW][128] norms of the current tile
+  uint32_t* pn_s = (uint32_t*)after;         // [EW][128] norms of the current tile
   const uint32_t b0 = smem_u32(bars);
   auto bar_q = [&](uint32_t i) { return b0 + 8 * i; };            // 0 loaded, 1 free
   auto bar_full = [&](uint32_t s) { return b0 + 8 * (2 + s); };
@@ -614,6 +614,8 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
     uint32_t* pn_w = pn_s + wid * 128;
     uint32_t buf = 0, tph = 0;
     uint32_t cnt = 0;
+    uint64_t tile = 0;          // the segment's list tile
+    uint32_t *lv = nullptr, *li = nullptr;  // its scores and ids, [kGtCap][ROWS]
     uint32_t thr = 0;       // the score a value must beat (int) or reach (float), as bits
     float err2 = 0.f;
     bool dead = true;       // no query, or given up
@@ -628,18 +630,20 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
         const uint32_t rr = wid * 32 + src;
         const uint32_t c = __shfl_sync(FULL, cnt, src);
         const float e2 = __shfl_sync(FULL, err2, src);
-        uint32_t v[2], id[2], rk[2] = {0, 0};
+        constexpr int PER = kGtCap / 32;
+        uint32_t v[PER], id[PER], rk[PER];
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
+        for (int j = 0; j < PER; j++) {
           const uint32_t e = lane + 32 * j;
           v[j] = e < c ? lv[e * ROWS + rr] : 0u;
           id[j] = e < c ? li[e * ROWS + rr] : 0u;
+          rk[j] = 0;
         }
 #pragma unroll 4
         for (uint32_t e = 0; e < c; e++) {
           const uint32_t ov = lv[e * ROWS + rr], oi = li[e * ROWS + rr];
 #pragma unroll
-          for (int j = 0; j < 2; j++) {
+          for (int j = 0; j < PER; j++) {
             const uint32_t a = gt_rank_bits<F32>(ov), b = gt_rank_bits<F32>(v[j]);
             rk[j] += (a > b || (a == b && oi < id[j])) ? 1u : 0u;
           }
@@ -647,7 +651,7 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
         uint32_t kth = 0;
         bool mine = false;
 #pragma unroll
-        for (int j = 0; j < 2; j++)
+        for (int j = 0; j < PER; j++)
           if (lane + 32 * j < c && rk[j] == g.k - 1) {
             mine = true;
             kth = v[j];
@@ -661,7 +665,7 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
         __syncwarp();
         uint32_t kept = 0;
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
+        for (int j = 0; j < PER; j++) {
           const bool keep = lane + 32 * j < c &&
                             (F32 ? __uint_as_float(v[j]) >= __uint_as_float(nthr) : rk[j] < g.k);
           if (keep) {
@@ -675,7 +679,7 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
           cnt = kept;
           if (who) thr = F32 ? __float_as_uint(fmaxf(__uint_as_float(thr), __uint_as_float(nthr)))
                              : (uint32_t)max((int)thr, (int)nthr);
-          if (kept > CAP - 8) {  // float: too many within the bound
+          if (kept > kGtCap - 8) {  // float: too many within the bound
             dead = true;
             cnt = 0;
           }
@@ -692,6 +696,10 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
     for (uint32_t t = 0; t < nt; t++, next_step()) {
       const uint64_t q = (uint64_t)qt * ROWS + r;
       if (t == 0 || bt == 0) {
+        const uint64_t seg = blockIdx.x - ((uint64_t)qt * g.btiles) / g.per;
+        tile = g.list0 / ROWS + qt * g.segs + seg;
+        lv = g.ent_v + tile * kGtCap * ROWS;
+        li = g.ent_i + tile * kGtCap * ROWS;
         cnt = 0;
         dead = q >= g.nq;
         if (F32 && !dead) {
@@ -751,7 +759,7 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
                 cnt++;
               }
             __syncwarp();
-            compact(__ballot_sync(FULL, cnt > CAP - 8));
+            compact(__ballot_sync(FULL, cnt > kGtCap - 8));
           }
         }
       };
@@ -777,15 +785,7 @@ __global__ void __launch_bounds__(MTILES * 128 + 64, 1)
           gbest = 0;
         }
       } else if (t + 1 == nt || bt + 1 == g.btiles) {
-        // the segment's lists (a warp's 32 rows side by side)
-        compact(__ballot_sync(FULL, cnt > 0));
-        const uint64_t seg = blockIdx.x - ((uint64_t)qt * g.btiles) / g.per;
-        const uint64_t tile = g.list0 / ROWS + qt * g.segs + seg;
         g.cnt[tile * ROWS + r] = cnt;
-        for (uint32_t e = 0; e < cnt; e++) {
-          g.ent_v[(tile * kGtKeep + e) * ROWS + r] = lv[e * ROWS + r];
-          g.ent_i[(tile * kGtKeep + e) * ROWS + r] = li[e * ROWS + r];
-        }
         if (F32 && dead && q < g.nq) g.over[q] = 1u;
         __syncwarp();
       }
@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(256) k_gt_merge(IndexView ix, const uint8_t* q
       for (uint32_t b = 0; b < c; b += 32) {
         const uint32_t e = b + lane;
         const double v =
-            e < c ? -(double)__uint_as_float(ent_v[(tile * kGtKeep + e) * rows + r]) : INFINITY;
+            e < c ? -(double)__uint_as_float(ent_v[(tile * kGtCap + e) * rows + r]) : INFINITY;
         const double td = __shfl_sync(0xffffffffu, sd, k - 1);
         topk_insert(sd, si, k, v, e, v < td);
       }
@@ -906,8 +906,8 @@ __global__ void __launch_bounds__(256) k_gt_merge(IndexView ix, const uint8_t* q
     const uint32_t c = cnt[tile * rows + r];
     for (uint32_t b = 0; b < c; b += 32) {
       const uint32_t e = b + lane;
-      const uint32_t v = e < c ? ent_v[(tile * kGtKeep + e) * rows + r] : 0u;
-      const uint32_t iv = e < c ? ent_i[(tile * kGtKeep + e) * rows + r] : DD_NONE;
+      const uint32_t v = e < c ? ent_v[(tile * kGtCap + e) * rows + r] : 0u;
+      const uint32_t iv = e < c ? ent_i[(tile * kGtCap + e) * rows + r] : DD_NONE;
       if (F32) {
         uint32_t m = __ballot_sync(0xffffffffu, e < c && __uint_as_float(v) >= cut);
         for (; m; m &= m - 1) {

@@ -83,3 +83,34 @@ def test_several_slabs_of_float_rows(oracle_mod):
     q = rng.standard_normal((20, 5), dtype=np.float32)
     base[1_050_000:1_050_020] = q  # the nearest ones lie in the second slab
     _check(oracle_mod, base, q, "l2", (10,))
+
+
+@pytest.mark.parametrize("metric", ["l2", "mips"])
+@pytest.mark.parametrize("dtype,d", [("u8", 64), ("i8", 200), ("f32", 24)])
+def test_lists_that_fill_up(oracle_mod, metric, dtype, d):
+    """31 tiles (no sample), several a CTA, the rows ever nearer: every value passes its
+    query's threshold until the list is compacted."""
+    rng = np.random.default_rng(d)
+    n, nq = 31 * 128 - 5, 2_600
+    t = {"u8": np.uint8, "i8": np.int8, "f32": np.float32}[dtype]
+    base = np.zeros((n, d), t)
+    base += (np.arange(n) * (100.0 / n)).astype(t)[:, None]
+    base[:, 0] = rng.integers(0, 100, n)
+    q = (100 + rng.integers(0, 20, (nq, d))).astype(t)
+    _check(oracle_mod, base, q, metric, (32, 5))
+
+
+def test_more_queries_than_one_workspace():
+    rng = np.random.default_rng(12)
+    n, nq, d, k = 4_000, 1_500_001, 4, 3
+    base = rng.integers(0, 256, (n, d)).astype(np.uint8)
+    q = rng.integers(0, 256, (nq, d)).astype(np.uint8)
+    gi = GpuIndex(base.dtype, "l2", n, d, 8)
+    gi.upload_points(base)
+    ids, ds = gi.groundtruth(q, k)
+    for pick in (slice(0, 1000), slice(nq // 2 - 500, nq // 2 + 500),
+                 slice(nq // 4 - 500, nq // 4 + 500), slice(nq - 1000, nq)):
+        wi, wd = gi.groundtruth(q[pick], k)
+        np.testing.assert_array_equal(ids[pick], wi)
+        np.testing.assert_array_equal(ds[pick], wd)
+    gi.close()
