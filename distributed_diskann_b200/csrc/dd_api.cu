@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <fstream>
 #include <mutex>
@@ -87,12 +88,11 @@ struct dd_index {
   uint64_t qhash_words = 0;
   uint32_t* qev = nullptr;    // evicted lists of the query searches
   uint64_t qev_words = 0;
-  // host calls (search, beam search, prune, ground truth): one device buffer
-  // and one pinned staging buffer, kept up to kIoKeepBytes / kPinKeepBytes
+  // host calls (search, beam search, prune, ground truth): one device buffer,
+  // kept up to kIoKeepBytes
   uint8_t* io = nullptr;
   uint64_t io_bytes = 0;
-  uint8_t* pin = nullptr;
-  uint64_t pin_bytes = 0;
+  bool host_call = false;  // a host call has been staged before
   std::vector<std::pair<uint64_t, LaunchPlan>> qplans;  // query CTA shapes by layout
   // sharded build: the launch shapes and parameters set by dd_shard_begin
   bool shard_ready = false;
@@ -182,9 +182,9 @@ void dfree(void* p) {
 // The buffers of one host call.  Allocating and freeing device memory in every
 // call cost 70 us (small calls) to several ms (megabytes, and cudaFree waits for
 // the device), and each copy from or to pageable memory 15 us or more: the
-// device buffer stays with the handle, the inputs go up in one copy from pinned
-// staging and the results come down in one (up to kPinKeepBytes; larger calls
-// copy each array directly).  512 robustPrune tasks 2.4 -> 0.7 ms, one query 450
+// device buffer stays with the handle, the inputs go up in one copy from a
+// staging buffer and the results come down in one (up to kPinKeepBytes; larger
+// calls copy each array directly).  512 robustPrune tasks 2.4 -> 0.7 ms, one query 450
 // -> 400 us, 30,000 queries of 100 bytes 18 -> 9.6 ms.
 constexpr uint64_t kIoKeepBytes = 1ull << 30, kPinKeepBytes = 64ull << 20;
 
@@ -207,23 +207,102 @@ int ensure_io(dd_index* h, uint64_t bytes) {
   return DD_OK;
 }
 
-// pinned staging of at least `bytes`; null when the call is too large for it
-uint8_t* pinned(dd_index* h, uint64_t bytes) {
-  if (bytes > kPinKeepBytes) return nullptr;
-  if (bytes > h->pin_bytes) {
-    if (h->pin) cudaFreeHost(h->pin);
-    h->pin = nullptr;
-    h->pin_bytes = 0;
-    const uint64_t want = std::max<uint64_t>(bytes, 1u << 20);
-    if (cudaMallocHost((void**)&h->pin, want) != cudaSuccess) {
-      cudaGetLastError();
-      h->pin = nullptr;
-      return nullptr;
-    }
-    h->pin_bytes = want;
+// Idle pinned buffers, at most kPinKeepBytes of them, for the host calls of all
+// handles; the last handle's end frees them.
+struct PinPool {
+  struct Buf {
+    uint8_t* p;
+    uint64_t bytes;
+  };
+  std::mutex mu;
+  std::vector<Buf> idle;
+  uint64_t handles = 0;
+
+  void drop(size_t i) {
+    cudaFreeHost(idle[i].p);
+    idle.erase(idle.begin() + i);
   }
-  return h->pin;
+  void open() {
+    std::lock_guard<std::mutex> g(mu);
+    handles++;
+  }
+  void close() {
+    std::lock_guard<std::mutex> g(mu);
+    if (--handles == 0)
+      while (!idle.empty()) drop(idle.size() - 1);
+  }
+  // the smallest that fits
+  Buf get(uint64_t bytes) {
+    std::lock_guard<std::mutex> g(mu);
+    size_t best = idle.size();
+    for (size_t i = 0; i < idle.size(); i++)
+      if (idle[i].bytes >= bytes && (best == idle.size() || idle[i].bytes < idle[best].bytes)) best = i;
+    if (best == idle.size()) return {nullptr, 0};
+    const Buf b = idle[best];
+    idle.erase(idle.begin() + best);
+    return b;
+  }
+  // beyond the bound the smallest go first: a larger one serves their calls too
+  void put(Buf b) {
+    std::lock_guard<std::mutex> g(mu);
+    idle.push_back(b);
+    uint64_t total = 0;
+    for (const Buf& x : idle) total += x.bytes;
+    while (total > kPinKeepBytes) {
+      size_t s = 0;
+      for (size_t i = 1; i < idle.size(); i++)
+        if (idle[i].bytes < idle[s].bytes) s = i;
+      total -= idle[s].bytes;
+      drop(s);
+    }
+  }
+};
+PinPool& pin_pool() {
+  static PinPool* pool = new PinPool;  // no destructor: the CUDA runtime may be gone by then
+  return *pool;
 }
+
+// Host staging of one call, at least `bytes`; p is null when the call is too
+// large for it.  A handle's first call takes pageable memory (still one copy each
+// way) unless a pinned buffer is idle: allocating one takes 1 to 5 ms, which only
+// later calls win back (a fresh handle's first call of one query: 1.9 ms with the
+// allocation, 0.5 ms without; 0.65 ms with a buffer and a copy for each array).
+class Staging {
+ public:
+  uint8_t* p = nullptr;
+
+  Staging(dd_index* h, uint64_t bytes) : h_(h) {
+    if (bytes > kPinKeepBytes) return;
+    buf_ = pin_pool().get(bytes);
+    p = buf_.p;
+    if (!p && h->host_call) {
+      uint64_t want = 1u << 20;
+      while (want < bytes) want *= 2;
+      if (cudaHostAlloc((void**)&p, want, cudaHostAllocPortable) == cudaSuccess) {
+        buf_ = {p, want};
+      } else {
+        cudaGetLastError();
+        p = nullptr;
+      }
+    } else if (!p) {
+      heap_ = (uint8_t*)std::malloc(std::max<uint64_t>(bytes, 1));
+      p = heap_;
+    }
+    h->host_call = true;
+  }
+  ~Staging() {
+    if (p) cudaStreamSynchronize(h_->stream);  // an error may leave a copy in flight
+    std::free(heap_);
+    if (buf_.p) pin_pool().put(buf_);
+  }
+  Staging(const Staging&) = delete;
+  Staging& operator=(const Staging&) = delete;
+
+ private:
+  dd_index* h_;
+  PinPool::Buf buf_{nullptr, 0};
+  uint8_t* heap_ = nullptr;
+};
 
 void release_io(dd_index* h) {
   if (h->io_bytes <= kIoKeepBytes) return;
@@ -725,6 +804,7 @@ int dd_create(int dtype, int metric, uint64_t n, uint32_t d, uint32_t R, int dev
   if (R > kMaxRp) return DD_ERR_UNSUPPORTED;
   if ((uint64_t)d * esize(dtype) > 1024) return DD_ERR_UNSUPPORTED;
   h = new dd_index();
+  pin_pool().open();
   h->dtype = dtype;
   h->metric = metric;
   h->n = n;
@@ -771,13 +851,13 @@ int dd_destroy(dd_index* h) {
   dfree(h->qhash);
   dfree(h->qev);
   dfree(h->io);
-  if (h->pin) cudaFreeHost(h->pin);
   if (h->gexec) cudaGraphExecDestroy(h->gexec);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   for (cudaStream_t a : h->fork.aux)
     if (a) cudaStreamDestroy(a);
   for (cudaEvent_t e : {h->fork.forked, h->fork.joined[0], h->fork.joined[1]})
     if (e) cudaEventDestroy(e);
+  pin_pool().close();
   delete h;
   return DD_OK;
 }
@@ -1437,39 +1517,54 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
     launch_bin_queries(L_per_query, nq, k, Lmax, h->qcls, counts, h->stream);
     h->launches++;
   }
+  // the scratch of the largest class is allocated before the first launch: a
+  // class that needs more would free what the one before it still uses
+  struct ClassRun {
+    int c, grid;
+    uint32_t L;
+    bool hglob;
+    WarpLayout lay;
+    LaunchPlan plan;
+  };
+  ClassRun runs[kQueryClasses];
+  int nruns = 0;
+  uint64_t warps = 0, hwords = 0;
   for (int c = query_class(Lmax); c >= 0; c--) {
     if (!((classes >> c) & 1u)) continue;
     if ((16u << c) < k && c < query_class(Lmax)) break;  // no valid beam width below k
-    const uint32_t Lc = std::min<uint32_t>(16u << c, Lmax);
+    ClassRun& r = runs[nruns++];
+    r.c = c;
+    r.L = std::min<uint32_t>(16u << c, Lmax);
     // seen tables above 16 KB (beam widths above 128) would cap the resident
     // queries per SM by shared memory: they go to one global slice per warp
-    const bool hglob = hash_table_bytes(hash_bits_for(Lc), use_h24(h)) > 16384;
-    WarpLayout lc = make_search_layout(h->d, h->dtype, h->metric, Lc, h->Rp, 2 * Lc + 64, false,
-                                       use_h24(h), false, true, hglob);
-    const LaunchPlan plan = query_plan(h, lc, Lc);
+    r.hglob = hash_table_bytes(hash_bits_for(r.L), use_h24(h)) > 16384;
+    r.lay = make_search_layout(h->d, h->dtype, h->metric, r.L, h->Rp, 2 * r.L + 64, false,
+                               use_h24(h), false, true, r.hglob);
+    r.plan = query_plan(h, r.lay, r.L);
+    const int wpc = r.plan.warps_per_cta;
+    r.grid = (int)std::min<uint64_t>((nq + wpc - 1) / wpc,
+                                     (uint64_t)r.plan.blocks_per_sm * h->sm_count);
+    warps = std::max(warps, (uint64_t)r.grid * wpc);
+    if (r.hglob) hwords = std::max(hwords, (uint64_t)r.grid * wpc * r.lay.hash_words);
+  }
+  int rc = ev_slices(warps);
+  if (rc) return rc;
+  if (hwords > h->qhash_words) {
+    dfree(h->qhash);
+    h->qhash = nullptr;
+    h->qhash_words = 0;
+    CK(dalloc(&h->qhash, hwords));
+    h->qhash_words = hwords;
+  }
+  for (int i = 0; i < nruns; i++) {
+    const ClassRun& r = runs[i];
     QueryArgs qc = qa;
-    qc.Lmax = Lc;
-    qc.cls_items = one ? nullptr : h->qcls + (uint64_t)c * nq;
-    qc.cls_count = one ? nullptr : counts + c;
-    qc.cls_queue = queues + c;
-    const int wpc = plan.warps_per_cta;
-    const int grid = (int)std::min<uint64_t>((nq + wpc - 1) / wpc,
-                                             (uint64_t)plan.blocks_per_sm * h->sm_count);
-    int rc = ev_slices((uint64_t)grid * wpc);
-    if (rc) return rc;
-    qc.ev_scratch = qa.ev_scratch;
-    if (hglob) {
-      const uint64_t words = (uint64_t)grid * wpc * lc.hash_words;
-      if (words > h->qhash_words) {
-        dfree(h->qhash);
-        h->qhash = nullptr;
-        h->qhash_words = 0;
-        CK(dalloc(&h->qhash, words));
-        h->qhash_words = words;
-      }
-      qc.hash_scratch = h->qhash;
-    }
-    launch_query(ixq, qc, lc, wpc, grid, h->stream);
+    qc.Lmax = r.L;
+    qc.cls_items = one ? nullptr : h->qcls + (uint64_t)r.c * nq;
+    qc.cls_count = one ? nullptr : counts + r.c;
+    qc.cls_queue = queues + r.c;
+    if (r.hglob) qc.hash_scratch = h->qhash;
+    launch_query(ixq, qc, r.lay, r.plan.warps_per_cta, r.grid, h->stream);
     h->launches++;
   }
   CK(cudaGetLastError());
@@ -1507,7 +1602,8 @@ int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
   int rc = ensure_io(h, io.total);
   if (rc) return rc;
   uint8_t* dev = h->io;
-  uint8_t* pin = pinned(h, std::max(in_bytes, out_bytes));
+  const Staging staged(h, std::max(in_bytes, out_bytes));
+  uint8_t* const pin = staged.p;
   if (pin) {
     stage_rows(pin + o_q, ds, (const uint8_t*)queries, qstride, rb, nq);
     std::memcpy(pin + o_L, L_per_query, nq * 4);
@@ -1627,7 +1723,8 @@ int dd_robust_prune(dd_index* h, uint32_t ntasks, const uint32_t* p, const uint6
   int rc = ensure_io(h, io.total);
   if (rc) return rc;
   uint8_t* dev = h->io;
-  uint8_t* pin = pinned(h, std::max(in_bytes, out_bytes));
+  const Staging staged(h, std::max(in_bytes, out_bytes));
+  uint8_t* const pin = staged.p;
   cudaError_t e = cudaSuccess;
   if (pin) {
     std::memcpy(pin + o_off, offsets, (ntasks + 1) * 8ull);
@@ -1683,7 +1780,8 @@ static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint
   uint32_t* di = (uint32_t*)(h->io + o_i);
   float* dd = (float*)(h->io + o_d);
   uint8_t* work = h->io + ((o_w + 1023) & ~(uint64_t)1023);
-  uint8_t* pin = pinned(h, std::max<uint64_t>(nq * ds, nq * k * 8ull + 64));
+  const Staging staged(h, std::max<uint64_t>(nq * ds, nq * k * 8ull + 64));
+  uint8_t* const pin = staged.p;
   uint8_t* parts = nullptr;
   uint32_t *over = nullptr, nover = 0;
   bool ok = true;

@@ -1,4 +1,4 @@
-"""Host calls share one device and one pinned buffer per handle, and search only the
+"""Host calls keep one device buffer per handle and share pinned staging, and search only the
 beam-width classes a call holds: calls of growing and shrinking sizes, strided query
 rows, one and several classes, calls that fail in between, and prunes on both sides of
 the shared-memory limit must give what the oracle (or a fresh handle) gives."""
@@ -58,6 +58,35 @@ def test_calls_of_changing_size_on_one_handle(oracle_mod, dtype):
                             p(ds), None, None))
     np.testing.assert_array_equal(ids, gi.search(q[:50], 10, 40)[0])
     gi.close()
+
+
+def test_handles_of_several_threads_share_the_staging():
+    """Handles opened, called and closed by threads at once, calls of growing and
+    shrinking size: the answers of one handle used alone."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    both = D.gen_mixture_i8(6_000, 24, 20, 6)
+    base, q = both[:3_000], both[3_000:]
+    sizes = (1, 2_900, 40, 900, 3)
+
+    def answers(seed):
+        out = []
+        for again in range(2):
+            gi = GpuIndex(base.dtype, "l2", 3_000, 24, 16)
+            gi.upload_points(base)
+            gi.build(32, 1.2)
+            for nq in sizes[seed:] + sizes[:seed]:
+                r = gi.search(q[:nq], 5, 20)
+                out.append((nq, r[0].copy(), gi.groundtruth(q[:nq], 3)[0]))
+            gi.close()
+        return sorted(out, key=lambda r: r[0])
+
+    want = answers(0)
+    with ThreadPoolExecutor(4) as pool:
+        for got in pool.map(answers, range(4)):
+            for w, g in zip(want, got):
+                np.testing.assert_array_equal(w[1], g[1])
+                np.testing.assert_array_equal(w[2], g[2])
 
 
 @pytest.mark.parametrize("dtype,metric,d", [("u8", "l2", 128), ("i8", "mips", 20),
