@@ -503,7 +503,7 @@ def main():
                             device=dev)
         qres = {"nq": nq, "k": k, "cut": 1.35,
                 "groundtruth_s": t_gt,  # host wall time of dd_groundtruth, k = 32, copies included
-                "groundtruth_form": "tensor-core Gram tiles" if w.dtype != "f32" else "FP64"}
+                "groundtruth_form": "tensor-core tiles" + ("" if w.dtype != "f32" else ", FP64 re-rank")}
         for form in ("fast", "plain"):
             gi.set_search_mode(form)
             sweep = []
@@ -551,7 +551,7 @@ def main():
                                    f"L={w.L}, alpha={w.alpha} (full batched build per step)",
                        "n": n, "d": w.d, "R": w.R, "L": w.L, "alpha": w.alpha,
                        "form": "fast (INT8 tensor-core prune tiles, set-associative seen "
-                               "filter and register step merges in the build search, "
+                               "filter and keyed-frontier step merges in the build search, "
                                "persistent work-queue kernels, CUDA-graph build replay, "
                                "autotuned CTA shapes); graph bit-exact vs the reference build",
                        "l2_flush": "inputs larger than L2 (points + graph > 126 MB)",
