@@ -1416,7 +1416,8 @@ LaunchPlan query_plan(dd_index* h, const WarpLayout& lay, uint32_t L) {
 }
 
 // dd_search_device; classes: the beam-width classes that may hold a query (bit
-// per class; all when the widths are only known on the device)
+// per class; kAllQueryClasses when the widths are only known on the device)
+constexpr uint32_t kAllQueryClasses = ~0u;
 int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
                      const uint32_t* L_per_query, uint32_t Lmax, uint32_t k, double cut,
                      uint64_t limit, uint32_t degree_limit, uint32_t start, int skip_self,
@@ -1510,13 +1511,7 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   }
   ixq.fgroup_lg = fast_fgroup(h);
   CK(cudaMemsetAsync(counts, 0, (2 * kQueryClasses + 1) * 4, h->stream));
-  // one class: every query is its, no list needed
-  const bool one = (classes & (classes - 1)) == 0;
-  h->launches = 0;
-  if (!one) {
-    launch_bin_queries(L_per_query, nq, k, Lmax, h->qcls, counts, h->stream);
-    h->launches++;
-  }
+  const bool known = classes != kAllQueryClasses;
   // the scratch of the largest class is allocated before the first launch: a
   // class that needs more would free what the one before it still uses
   struct ClassRun {
@@ -1546,6 +1541,22 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
                                      (uint64_t)r.plan.blocks_per_sm * h->sm_count);
     warps = std::max(warps, (uint64_t)r.grid * wpc);
     if (r.hglob) hwords = std::max(hwords, (uint64_t)r.grid * wpc * r.lay.hash_words);
+    // a call whose queries are all resident at once in the widest layout takes
+    // one launch of it: the classes one after another add their latencies (1500
+    // host queries of L = 10 to 200 on 1M x 128 uint8 2.99 -> 1.37 ms, 100 of them
+    // 2.13 -> 0.90).  Not above 256, where narrow queries would lose their keyed
+    // form, and not when the widths are unknown here: narrow queries alone are
+    // slower in a wide layout (1500 of L = 50 for a bound of 200 530 -> 614 us).
+    if (nruns == 1 && known && r.L <= 256 &&
+        nq <= (uint64_t)r.plan.blocks_per_sm * h->sm_count * wpc)
+      break;
+  }
+  // one launch: every query is its, no list needed
+  const bool one = nruns == 1 && known;
+  h->launches = 0;
+  if (!one) {
+    launch_bin_queries(L_per_query, nq, k, Lmax, h->qcls, counts, h->stream);
+    h->launches++;
   }
   int rc = ev_slices(warps);
   if (rc) return rc;
@@ -1578,7 +1589,7 @@ int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
                      uint64_t limit, uint32_t degree_limit, uint32_t start, int skip_self,
                      uint32_t* ids, float* dists, uint32_t* visited, uint32_t* cmps) {
   return search_on_device(h, queries, nq, qstride, L_per_query, Lmax, k, cut, limit, degree_limit,
-                          start, skip_self, ids, dists, visited, cmps, (1u << kQueryClasses) - 1);
+                          start, skip_self, ids, dists, visited, cmps, kAllQueryClasses);
 }
 
 int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
