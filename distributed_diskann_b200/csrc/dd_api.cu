@@ -1483,7 +1483,7 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
                                              (uint64_t)plan.blocks_per_sm * h->sm_count);
     int rc = ev_slices((uint64_t)grid * wpc);
     if (rc) return rc;
-    launch_query(view(h), qa, lay, wpc, grid, h->stream);
+    launch_query(view(h), qa, lay, wpc, grid, false, h->stream);
     h->launches = 1;
     CK(cudaGetLastError());
     return DD_OK;
@@ -1523,7 +1523,12 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   };
   ClassRun runs[kQueryClasses];
   int nruns = 0;
-  uint64_t warps = 0, hwords = 0;
+  // Classes run in groups of kLanes whose launches overlap: the next one's CTAs
+  // take the places that the tail of the one before leaves (launch_query), the
+  // widest class first.  Each has its own scratch; the first of a group waits for
+  // the group before.
+  constexpr int kLanes = 3;
+  uint64_t warps[kLanes] = {}, hwords[kLanes] = {};
   for (int c = query_class(Lmax); c >= 0; c--) {
     if (!((classes >> c) & 1u)) continue;
     if ((16u << c) < k && c < query_class(Lmax)) break;  // no valid beam width below k
@@ -1539,8 +1544,9 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
     const int wpc = r.plan.warps_per_cta;
     r.grid = (int)std::min<uint64_t>((nq + wpc - 1) / wpc,
                                      (uint64_t)r.plan.blocks_per_sm * h->sm_count);
-    warps = std::max(warps, (uint64_t)r.grid * wpc);
-    if (r.hglob) hwords = std::max(hwords, (uint64_t)r.grid * wpc * r.lay.hash_words);
+    const int s = (nruns - 1) % kLanes;
+    warps[s] = std::max(warps[s], (uint64_t)r.grid * wpc);
+    if (r.hglob) hwords[s] = std::max(hwords[s], (uint64_t)r.grid * wpc * r.lay.hash_words);
     // a call whose queries are all resident at once in the widest layout takes
     // one launch of it: the classes one after another add their latencies (1500
     // host queries of L = 10 to 200 on 1M x 128 uint8 2.99 -> 1.37 ms, 100 of them
@@ -1558,24 +1564,31 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
     launch_bin_queries(L_per_query, nq, k, Lmax, h->qcls, counts, h->stream);
     h->launches++;
   }
-  int rc = ev_slices(warps);
-  if (rc) return rc;
-  if (hwords > h->qhash_words) {
+  const uint64_t hsum = hwords[0] + hwords[1] + hwords[2];
+  int rc = ev_slices(warps[0] + warps[1] + warps[2]);
+  if (!rc && hsum > h->qhash_words) {
     dfree(h->qhash);
     h->qhash = nullptr;
     h->qhash_words = 0;
-    CK(dalloc(&h->qhash, hwords));
-    h->qhash_words = hwords;
+    CK(dalloc(&h->qhash, hsum));
+    h->qhash_words = hsum;
   }
+  if (rc) return rc;
   for (int i = 0; i < nruns; i++) {
     const ClassRun& r = runs[i];
+    const int s = i % kLanes;
     QueryArgs qc = qa;
     qc.Lmax = r.L;
     qc.cls_items = one ? nullptr : h->qcls + (uint64_t)r.c * nq;
     qc.cls_count = one ? nullptr : counts + r.c;
     qc.cls_queue = queues + r.c;
+    qc.ev_scratch = qa.ev_scratch;
     if (r.hglob) qc.hash_scratch = h->qhash;
-    launch_query(ixq, qc, r.lay, r.plan.warps_per_cta, r.grid, h->stream);
+    for (int t = 0; t < s; t++) {
+      qc.ev_scratch += warps[t] * qa.ev_cap;
+      if (r.hglob) qc.hash_scratch += hwords[t];
+    }
+    launch_query(ixq, qc, r.lay, r.plan.warps_per_cta, r.grid, s != 0, h->stream);
     h->launches++;
   }
   CK(cudaGetLastError());

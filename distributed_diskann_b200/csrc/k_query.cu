@@ -41,6 +41,7 @@ __device__ __forceinline__ SearchSmem carve_query(uint8_t* base, const WarpLayou
 template <int DT, int MT, int FPL, int CPL>
 __global__ void __launch_bounds__(512) k_query(IndexView ix, QueryArgs qa, WarpLayout lay) {
   extern __shared__ uint4 smem_raw[];
+  cudaTriggerProgrammaticLaunchCompletion();  // the next class may start where there is room
   const uint32_t wpc = blockDim.x >> 5, wic = threadIdx.x >> 5, lane = lane_id();
   const uint64_t gw = (uint64_t)blockIdx.x * wpc + wic;
   // large seen tables (beam widths above 128) live in this warp's global slice
@@ -104,6 +105,9 @@ __global__ void __launch_bounds__(512) k_query(IndexView ix, QueryArgs qa, WarpL
     }
     __syncwarp();
   }
+  // an overlapped class ends after the one before it, so that what follows on
+  // the stream finds both done
+  cudaGridDependencySynchronize();
 }
 
 __global__ void k_bin_queries(const uint32_t* Ls, uint64_t nq, uint32_t k, uint32_t Lvalid,
@@ -167,12 +171,32 @@ LaunchPlan plan_query(const IndexView& ix, const WarpLayout& lay, uint32_t Lmax)
   return p;
 }
 
+// overlap: the launch may start once every CTA of the k_query launch before it on
+// the stream has started (nothing it reads comes from there: the class lists were
+// complete when that one began, and each has its own scratch).  A class's last
+// searches leave most of the GPU idle, and a call of mixed widths had one such
+// tail per class.  Measured on B200, 10,000 queries of L = 10 to 200 mixed, classes
+// one after another against overlapped: 10M x 128 uint8 4.89 -> 3.67 ms, 1M 3.57 ->
+// 2.64, 100k x 64 f32 3.11 -> 2.32; calls of one width the same.  Forked streams
+// overlap the classes a little more (2.43 and 2.14 ms), but a narrow class may
+// then start first and take the places of the widest: calls of L = 200 alone on
+// 10M took 7.3 or 11.5 ms instead of 7.5.
 void launch_query(const IndexView& ix, const QueryArgs& qa, const WarpLayout& lay, int wpc,
-                  int grid, cudaStream_t st) {
+                  int grid, bool overlap, cudaStream_t st) {
   size_t sm = (size_t)lay.total * wpc;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(wpc * 32);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = overlap ? 1 : 0;
 #define CALL4(DT, MT, F, C)                                                          \
   set_smem(k_query<DT, MT, F, C>, sm);                                               \
-  k_query<DT, MT, F, C><<<grid, wpc * 32, sm, st>>>(ix, qa, lay);
+  cudaLaunchKernelEx(&cfg, k_query<DT, MT, F, C>, ix, qa, lay);
 #define CALL(DT, MT) DD_DISPATCH_FC(qa.Lmax, ix.Rp, DT, MT, CALL4)
   DD_DISPATCH_DM(ix.dtype, ix.metric, CALL);
 #undef CALL

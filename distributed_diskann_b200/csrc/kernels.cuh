@@ -214,7 +214,7 @@ void launch_bin_queries(const uint32_t* Ls, uint64_t nq, uint32_t k, uint32_t Lv
                         uint32_t* items, uint32_t* counts, cudaStream_t st);
 LaunchPlan plan_query(const IndexView& ix, const WarpLayout& lay, uint32_t Lmax);
 void launch_query(const IndexView& ix, const QueryArgs& qa, const WarpLayout& lay,
-                  int warps_per_cta, int grid, cudaStream_t st);
+                  int warps_per_cta, int grid, bool overlap, cudaStream_t st);
 
 // beam_search with full frontier + visited outputs (kernel-level parity tests)
 struct BeamArgs {

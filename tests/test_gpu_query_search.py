@@ -62,3 +62,45 @@ def test_query_widths_and_repeated_ids(oracle_mod, dtype, metric, d, R, repeats)
             found = np.isfinite(ds)
             np.testing.assert_array_equal(ids[found], oi[found])
     gi.close()
+
+
+@pytest.mark.parametrize("dtype", ["u8", "f32"])
+@pytest.mark.parametrize("nq,widths", [
+    (3, (10, 200)), (900, (10, 20, 50, 100, 200)),       # one launch of the widest layout
+    (9_000, (10, 20, 50, 100, 200)),                     # overlapped classes, two groups
+    (4_000, (500, 10, 300, 130, 70, 40, 20, 12)),        # every class
+])
+def test_mixed_widths_in_one_call(dtype, nq, widths):
+    """One call of several beam widths, from the host and on the device (where the
+    widths are unknown to the launch), against a call of each width alone."""
+    import torch
+
+    gen = {"f32": D.gen_mixture_f32, "u8": D.gen_skewed_u8}[dtype]
+    both = gen(4_000 + nq, 32, 15, 4)
+    base, q = both[:4_000], np.ascontiguousarray(both[4_000:])
+    gi = GpuIndex(base.dtype, "l2", 4_000, 32, 32)
+    gi.upload_points(base)
+    gi.build(64, 1.2)
+    Ls = np.resize(np.asarray(widths, np.uint32), nq)
+    want = [None, np.zeros((nq, 10), np.float32), np.zeros(nq, np.uint32), np.zeros(nq, np.uint32)]
+    want[0] = np.zeros((nq, 10), np.uint32)
+    for w in widths:
+        for a, b in zip(want, gi.search(q, 10, int(w))):
+            a[Ls == w] = b[Ls == w]
+    for _ in range(2):
+        for a, b in zip(want, gi.search(q, 10, Ls)):
+            np.testing.assert_array_equal(a, b)
+    dq = torch.from_numpy(q).cuda()
+    dL = torch.from_numpy(Ls.view(np.int32)).cuda()
+    out = [torch.zeros((nq, 10), dtype=torch.int32, device="cuda"),
+           torch.zeros((nq, 10), device="cuda"),
+           torch.zeros(nq, dtype=torch.int32, device="cuda"),
+           torch.zeros(nq, dtype=torch.int32, device="cuda")]
+    torch.cuda.synchronize()
+    gi.search_device(dq.data_ptr(), nq, dq.stride(0) * dq.element_size(), dL.data_ptr(),
+                     max(widths), 10, out[0].data_ptr(), out[1].data_ptr(),
+                     vis_ptr=out[2].data_ptr(), cmps_ptr=out[3].data_ptr())
+    torch.cuda.synchronize()
+    for a, b in zip(want, out):
+        np.testing.assert_array_equal(a.view(np.int32), b.cpu().numpy().view(np.int32))
+    gi.close()
