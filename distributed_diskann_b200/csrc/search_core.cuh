@@ -1242,7 +1242,8 @@ __device__ SearchOut warp_beam_search(const SearchParams& P, const SearchSmem& S
 //
 //  * A frontier entry is one 64-bit key: the distance's bits in ascending
 //    order, then id << 1 | visited; the array is padded with all-ones keys, so
-//    a lower bound is a fixed number of (load, compare, add) steps.
+//    a lower bound is a fixed number of (load, compare, add) steps
+//    (key_lower_bound).
 //  * The unvisited positions are a bitmap (one bit per entry, the same words in
 //    every lane): the next node and the one after it are its first two bits.
 //  * The kept candidates' final slots (lower bound + rank among them) are
@@ -1255,7 +1256,9 @@ __device__ SearchOut warp_beam_search(const SearchParams& P, const SearchSmem& S
 // Rows hold no repeated id and the search has no k-cut (rows_without_repeats),
 // so the frontier is a set and a step's candidates are distinct.  More than 32
 // candidates are merged 32 at a time: a union trimmed to L twice is the union
-// trimmed once, and the blocks pushed off still descend.
+// trimmed once, and the blocks pushed off still descend.  (All of a step's
+// candidates beat the cutoff it began with, but the ones from the 33rd on need
+// not beat the last entry that the first ones left: see key_lower_bound.)
 // ---------------------------------------------------------------------------
 template <int MT>
 __device__ __forceinline__ uint32_t dist_order(float d) {  // monotone
@@ -1267,6 +1270,50 @@ template <int MT>
 __device__ __forceinline__ float order_dist(uint32_t o) {
   if (MT == DD_L2) return __uint_as_float(o);
   return __uint_as_float((o & 0x80000000u) ? o ^ 0x80000000u : ~o);
+}
+
+// The first of a frontier's NF slots whose key is not below c, and the entry
+// there; the steps add up to NF - 1, so the last slot stands for "beyond it"
+// too, when all NF entries are below c.  Candidate c is new to the frontier and
+// nearer than its end iff the entry is above c | 1: it is c or c | 1 when the
+// frontier holds the candidate, and below c when the array is full of nearer
+// entries, where c would be trimmed at once.  (All ones, no candidate, is never
+// below an entry.)
+template <uint32_t NF>
+__device__ __forceinline__ uint32_t key_lower_bound(const unsigned long long* fr,
+                                                    unsigned long long c,
+                                                    unsigned long long* at) {
+  uint32_t lo = 0;
+#pragma unroll
+  for (uint32_t step = NF / 2; step; step >>= 1)
+    if (fr[lo + step - 1] < c) lo += step;
+  *at = fr[lo];
+  return lo;
+}
+
+// Opens the candidate slots M (bits, `upto` of them) of a frontier that will
+// have new_n entries: slot s holds a candidate, or the old entry s - (candidate
+// slots below s).  Every slot down to the first changed word is rewritten; a
+// word's old entries lie in it and in the words below, so from the last word on
+// each is read before anything it needs is written.  U: the unvisited positions,
+// candidates counted as unvisited.
+template <int FPL>
+__device__ __forceinline__ void open_slots(unsigned long long* fr, const uint32_t (&M)[FPL],
+                                           uint32_t upto, uint32_t new_n, uint32_t (&U)[FPL]) {
+  const uint32_t lane = lane_id(), lt = lanemask_lt();
+#pragma unroll
+  for (int t = FPL - 1; t >= 0; t--) {
+    if (upto) {
+      const uint32_t below = upto - __popc(M[t]);
+      const uint32_t s = 32 * t + lane;
+      const bool in = s < new_n, isc = (M[t] >> lane) & 1u;
+      const unsigned long long v = in ? fr[s - below - __popc(M[t] & lt)] : ~0ull;
+      __syncwarp();
+      if (in && !isc) fr[s] = v;
+      U[t] = __ballot_sync(0xffffffffu, in && (isc || !(v & 1ull)));
+      upto = below;
+    }
+  }
 }
 
 template <int DT, int MT, int FPL, int CPL>
@@ -1384,12 +1431,9 @@ __device__ SearchOut warp_build_search(const SearchParams& P, const SearchSmem& 
     for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
       // ---- one candidate per lane: lower bound in the frontier, and whether it is there
       u64 c = c0 + lane < nc ? cand[c0 + lane] : ~0ull;
-      uint32_t lo = 0;
-#pragma unroll
-      for (uint32_t step = NF / 2; step; step >>= 1)
-        if (fr[lo + step - 1] < c) lo += step;
-      const u64 at = fr[lo];
-      const bool keep = c != ~0ull && (at >> 1) != (c >> 1);
+      u64 at;
+      const uint32_t lo = key_lower_bound<NF>(fr, c, &at);
+      const bool keep = at > (c | 1ull);
       const uint32_t K = __ballot_sync(FULL, keep);
       const bool last_group = c0 + 32 >= nc;
       if (!K) {
@@ -1432,25 +1476,10 @@ __device__ SearchOut warp_build_search(const SearchParams& P, const SearchSmem& 
           }
         }
       }
-      // ---- every slot down to the first changed word: a word's old entries lie
-      // in it and in the words below, so from the last word on each is read
-      // before anything it needs is written
-      uint32_t upto = 0;  // candidate slots in words 0 .. t
+      uint32_t slots = 0;
 #pragma unroll
-      for (int t = 0; t < FPL; t++) upto += __popc(M[t]);
-#pragma unroll
-      for (int t = FPL - 1; t >= 0; t--) {
-        if (upto) {
-          const uint32_t below = upto - __popc(M[t]);
-          const uint32_t s = 32 * t + lane;
-          const bool in = s < new_n, isc = (M[t] >> lane) & 1u;
-          const u64 v = in ? fr[s - below - __popc(M[t] & lt)] : ~0ull;
-          __syncwarp();
-          if (in && !isc) fr[s] = v;
-          U[t] = __ballot_sync(FULL, in && (isc || !(v & 1ull)));
-          upto = below;
-        }
-      }
+      for (int t = 0; t < FPL; t++) slots += __popc(M[t]);
+      open_slots<FPL>(fr, M, slots, new_n, U);
       if (dst < new_n) fr[dst] = c;
       fr_n = new_n;
       __syncwarp();
@@ -1634,16 +1663,13 @@ __device__ bool warp_query_search(const SearchParams& P, const SearchSmem& S, ui
       u64 c = c0 + lane < nc ? cand[c0 + lane] : ~0ull;
       for (uint32_t e = 0; e < c0; e++)  // (more than 32 candidates) a copy in an earlier group
         if (__any_sync(FULL, cand[e] == c)) return false;
-      uint32_t lo = 0;
-#pragma unroll
-      for (uint32_t step = NF / 2; step; step >>= 1)
-        if (fr[lo + step - 1] < c) lo += step;
-      const u64 at = fr[lo];
-      const bool keep = c != ~0ull && (at >> 1) != (c >> 1);
+      u64 at;
+      const uint32_t lo = key_lower_bound<NF>(fr, c, &at);
+      const bool keep = at > (c | 1ull);
       const uint32_t K = __ballot_sync(FULL, keep);
       const bool last_group = c0 + 32 >= nc;
       // of two copies of an entry that the frontier holds, the second is kept
-      const bool held = c != ~0ull && !keep;
+      const bool held = c != ~0ull && (at >> 1) == (c >> 1);
       if (__popc(__ballot_sync(FULL, held)) > 1) {
         const uint32_t same = __match_any_sync(FULL, held ? lo32(c) : (lane << 1) | 1u);
         if (__any_sync(FULL, held && __popc(same) > 1)) return false;
@@ -1692,20 +1718,7 @@ __device__ bool warp_query_search(const SearchParams& P, const SearchSmem& S, ui
         if (off) evict(lane < off ? fr[fr_n - off + lane] : 0ull);
       }
       __syncwarp();
-      uint32_t upto = slots;
-#pragma unroll
-      for (int t = FPL - 1; t >= 0; t--) {
-        if (upto) {
-          const uint32_t below = upto - __popc(M[t]);
-          const uint32_t s = 32 * t + lane;
-          const bool in = s < new_n, isc = (M[t] >> lane) & 1u;
-          const u64 v = in ? fr[s - below - __popc(M[t] & lt)] : ~0ull;
-          __syncwarp();
-          if (in && !isc) fr[s] = v;
-          U[t] = __ballot_sync(FULL, in && (isc || !(v & 1ull)));
-          upto = below;
-        }
-      }
+      open_slots<FPL>(fr, M, slots, new_n, U);
       if (dst < new_n) fr[dst] = c;
       for (uint32_t b = ab; b; b &= b - 1) {
         const uint32_t d = __shfl_sync(FULL, dst, __ffs(b) - 1);
