@@ -334,23 +334,25 @@ int ensure_screen(dd_index* h) {
   return DD_OK;
 }
 
+int device_error(dd_index* h, uint32_t e) {
+  if (!e) return DD_OK;
+  std::string m = "device error:";
+  if (e & DD_EBAD_ID) m += " neighbour id out of range;";
+  if (e & DD_EVIS_CAP) m += " visited list exceeded its capacity (raise vcap);";
+  if (e & DD_ECAND_CAP) m += " a per-query beam width was 0, below k or above Lmax;";
+  if (e & DD_EDEGREE) m += " row degree exceeds R;";
+  if (e & DD_ESEG_CAP) m += " reverse-edge group exceeded the workspace;";
+  if (e & DD_ETIMEOUT) m += " a kernel's wait ran out;";
+  return fail(h, DD_ERR_DEVICE, "%s", m.c_str());
+}
+
 int check_error_word(dd_index* h, uint32_t* bits = nullptr) {
   uint32_t e = 0;
   CK(cudaMemcpyAsync(&e, h->err, 4, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   if (bits) *bits = e;
-  if (e) {
-    cudaMemsetAsync(h->err, 0, 4, h->stream);
-    std::string m = "device error:";
-    if (e & DD_EBAD_ID) m += " neighbour id out of range;";
-    if (e & DD_EVIS_CAP) m += " visited list exceeded its capacity (raise vcap);";
-    if (e & DD_ECAND_CAP) m += " a per-query beam width was 0, below k or above Lmax;";
-    if (e & DD_EDEGREE) m += " row degree exceeds R;";
-    if (e & DD_ESEG_CAP) m += " reverse-edge group exceeded the workspace;";
-    if (e & DD_ETIMEOUT) m += " a kernel's wait ran out;";
-    return fail(h, DD_ERR_DEVICE, "%s", m.c_str());
-  }
-  return DD_OK;
+  if (e) cudaMemsetAsync(h->err, 0, 4, h->stream);
+  return device_error(h, e);
 }
 
 // (floor, ceiling) rounds: src/bsp_index.hpp:162-166, 238-246 (identity order)
@@ -1807,7 +1809,7 @@ static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint
   const Staging staged(h, std::max<uint64_t>(nq * ds, nq * k * 8ull + 64));
   uint8_t* const pin = staged.p;
   uint8_t* parts = nullptr;
-  uint32_t *over = nullptr, nover = 0;
+  uint32_t *over = nullptr, left[2] = {0, 0};  // queries left, error bits
   bool ok = true;
   cudaError_t e = cudaSuccess;
   if (pin) {
@@ -1823,30 +1825,30 @@ static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint
     e = cudaGetLastError();
   }
   if (ok) {
-    auto download = [&]() {  // ids, distances and the word that counts what is left
+    auto download = [&]() {  // ids, distances and what is left
       if (pin) {
         e = cudaMemcpyAsync(pin, di, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(pin + nq * k * 4ull, dd, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(pin + nq * k * 8ull, over, 4, cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(pin + nq * k * 8ull, over, 8, cudaMemcpyDeviceToHost, h->stream);
       } else {
         e = cudaMemcpyAsync(ids, di, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(dists, dd, nq * k * 4ull, cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&nover, over, 4, cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(left, over, 8, cudaMemcpyDeviceToHost, h->stream);
       }
       if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
       if (e != cudaSuccess || !pin) return;
       std::memcpy(ids, pin, nq * k * 4ull);
       std::memcpy(dists, pin + nq * k * 4ull, nq * k * 4ull);
-      std::memcpy(&nover, pin + nq * k * 8ull, 4);
+      std::memcpy(left, pin + nq * k * 8ull, 8);
     };
     if (e == cudaSuccess) download();
-    if (e == cudaSuccess && nover) {  // float queries whose candidates the screen could not bound
-      const uint32_t left = nover;
+    if (const uint32_t todo = e == cudaSuccess ? left[0] : 0u) {
+      // float queries whose candidates the screen could not bound
       const uint64_t per = (uint64_t)groundtruth_exact_chunks(ix) * k * 12;
-      const uint32_t batch = (uint32_t)std::min<uint64_t>(left, std::max<uint64_t>(1, (256ull << 20) / per));
+      const uint32_t batch = (uint32_t)std::min<uint64_t>(todo, std::max<uint64_t>(1, (256ull << 20) / per));
       e = dalloc(&parts, batch * per);
-      for (uint32_t f = 0; e == cudaSuccess && f < left; f += batch) {
-        launch_groundtruth_exact(ix, dq, ds, nq, f, std::min(batch, left - f), k, di, dd, work,
+      for (uint32_t f = 0; e == cudaSuccess && f < todo; f += batch) {
+        launch_groundtruth_exact(ix, dq, ds, nq, f, std::min(batch, todo - f), k, di, dd, work,
                                  h->sm_count, parts, h->stream);
         e = cudaGetLastError();
       }
@@ -1858,7 +1860,7 @@ static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint
   release_io(h);
   CK(e);
   if (!ok) return fail(h, DD_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-  return check_error_word(h);
+  return device_error(h, left[1]);
 }
 
 int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride, uint32_t k,

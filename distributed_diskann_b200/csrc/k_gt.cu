@@ -231,7 +231,7 @@ static GtWork gt_work(const IndexView& ix, uint64_t nq, const GtShape& s) {
   };
   const uint64_t lists = s.nslabs * s.qtiles * s.segs * s.rows;
   w.zero0 = off;
-  w.scal = take(64);  // [0] largest |p|^2 bits, [1] overflowed queries
+  w.scal = take(64);  // [0] largest |p|^2 bits, [1] overflowed queries, [2] error bits
   w.over = take(4 * nq);
   w.cnt = take(4 * lists);
   w.gmax = take(s.groups ? 4ull * nq * kGtGroups : 0);
@@ -987,8 +987,9 @@ static void gt_launch(const GtShape& s, const CUtensorMap& qm, const CUtensorMap
 }
 
 // queries: nq device rows, qstride bytes apart (a multiple of 64), zero padded.
-// work: groundtruth_work_bytes.  *over (device, after the stream has run): how
-// many queries launch_groundtruth_exact must still compute.
+// work: groundtruth_work_bytes.  (*over)[0] (device, after the stream has run): how
+// many queries launch_groundtruth_exact must still compute; (*over)[1]: the
+// error bits of these launches (the index's word keeps what other calls left).
 bool launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qstride, uint64_t nq,
                         uint32_t k, uint32_t* ids, float* dists, uint8_t* work, int sm_count,
                         cudaStream_t st, uint32_t** over) {
@@ -1018,7 +1019,7 @@ bool launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qs
   g.cnt = (uint32_t*)(work + w.cnt);
   g.ent_v = (uint32_t*)(work + w.ent_v);
   g.ent_i = (uint32_t*)(work + w.ent_i);
-  g.err = ix.err;
+  g.err = scal + 2;
   g.gmax = (uint32_t*)(work + w.gmax);
   uint32_t* thr0 = (uint32_t*)(work + w.thr0);
   const uint32_t shape_bits = ((kGtTile >> 3) << 17) | ((128u >> 4) << 24);

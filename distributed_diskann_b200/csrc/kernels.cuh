@@ -257,9 +257,9 @@ void launch_prune_tasks_shared(const IndexView& ix, const PruneArgs& pa, uint64_
 
 // brute-force ground truth (k_gt.cu): device queries of stride qstride (a
 // multiple of 64, zero padded), a workspace of groundtruth_work_bytes; *over
-// names the device word that says how many float queries
-// launch_groundtruth_exact must still compute.  False: no tensor map could be
-// made.
+// names two device words: how many float queries launch_groundtruth_exact must
+// still compute, and the error bits of the launches.  False: no tensor map
+// could be made.
 uint64_t groundtruth_work_bytes(const IndexView& ix, uint64_t nq, uint32_t k, int sm_count);
 bool launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qstride, uint64_t nq,
                         uint32_t k, uint32_t* ids, float* dists, uint8_t* work, int sm_count,
