@@ -311,6 +311,14 @@ void release_io(dd_index* h) {
   h->io_bytes = 0;
 }
 
+// (a 2-D copy refuses such a stride, stage_rows does not look at it)
+int check_query_stride(dd_index* h, uint64_t qstride) {
+  const uint64_t rb = (uint64_t)h->d * esize(h->dtype);
+  if (qstride >= rb) return DD_OK;
+  return fail(h, DD_ERR_ARG, "query stride %llu < row bytes %llu", (unsigned long long)qstride,
+              (unsigned long long)rb);
+}
+
 // nq rows of rb bytes, qstride apart, into rows of ds bytes (zero padded) at dst
 void stage_rows(uint8_t* dst, uint64_t ds, const uint8_t* src, uint64_t qstride, uint64_t rb,
                 uint64_t nq) {
@@ -1613,6 +1621,8 @@ int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
               uint32_t* visited, uint32_t* cmps) {
   if (!h || !queries || !L_per_query || !ids || !dists) return DD_ERR_ARG;
   if (nq == 0) return DD_OK;
+  int rc = check_query_stride(h, qstride);
+  if (rc) return rc;
   CK(cudaSetDevice(h->device));
   const uint64_t rb = (uint64_t)h->d * esize(h->dtype), ds = h->stride;
   uint32_t Lmax = 0, classes = 0;
@@ -1625,7 +1635,7 @@ int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
   const uint64_t o_q = io.take(nq * ds), o_L = io.take(nq * 4), in_bytes = io.total;
   const uint64_t o_i = io.take(nq * k * 4ull), o_d = io.take(nq * k * 4ull), o_v = io.take(nq * 4),
                  o_c = io.take(nq * 4), out_bytes = io.total - in_bytes;
-  int rc = ensure_io(h, io.total);
+  rc = ensure_io(h, io.total);
   if (rc) return rc;
   uint8_t* dev = h->io;
   const Staging staged(h, std::max(in_bytes, out_bytes));
@@ -1868,6 +1878,7 @@ int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   if (!h || !queries || !ids || !dists) return DD_ERR_ARG;
   if (k == 0 || k > 32 || k > h->n) return fail(h, DD_ERR_UNSUPPORTED, "k must be in [1, 32]");
   if (nq == 0) return DD_OK;
+  if (const int rc = check_query_stride(h, qstride)) return rc;
   CK(cudaSetDevice(h->device));
   // the lists take 1 KB a query and segment: as many queries at a time as keep the
   // workspace within 2 GB, but at least 4096 (a float base is converted once a batch)

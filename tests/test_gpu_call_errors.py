@@ -1,5 +1,8 @@
-"""Whose errors a host call reports: a ground truth call answers for its own launches
-only."""
+"""What a host call refuses, and whose errors it reports: a ground truth call answers for
+its own launches only, and query rows closer together than their length are refused at
+every size."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -42,4 +45,24 @@ def test_ground_truth_leaves_an_earlier_search_error(oracle_mod, dtype):
     with pytest.raises(DDError, match="beam width"):
         gi.check_errors()
     gi.check_errors()
+    gi.close()
+
+
+@pytest.mark.parametrize("nq", [1, 50, 600_000])
+def test_query_rows_closer_than_their_length_are_refused(nq):
+    base = D.gen_skewed_u8(500, 120, 8, 5)  # 600,000 queries: more than a staging buffer holds
+    gi = GpuIndex(base.dtype, "l2", 500, 120, 16)
+    gi.upload_points(base)
+    gi.build(32, 1.2)
+    q = np.zeros((nq, 120), np.uint8)
+    Ls = np.full(nq, 20, np.uint32)
+    ids, ds = np.zeros((nq, 5), np.uint32), np.zeros((nq, 5), np.float32)
+    p = lambda a: C.c_void_p(a.ctypes.data)
+    for stride in (119, 60):
+        with pytest.raises(DDError):
+            gi._ck(gi.lib.dd_search(gi.h, p(q), nq, stride, p(Ls), 5, 1.35, 0, 0, 0, 1, p(ids),
+                                    p(ds), None, None))
+        with pytest.raises(DDError):
+            gi._ck(gi.lib.dd_groundtruth(gi.h, p(q), nq, stride, 5, p(ids), p(ds)))
+    gi.search(q, 5, 20)  # the handle goes on
     gi.close()
