@@ -391,17 +391,25 @@ std::vector<std::pair<uint64_t, uint64_t>> schedule(uint64_t n, uint64_t max_bui
 }
 
 int ensure_build_scratch(dd_index* h, uint64_t B) {
-  if (!h->counters) {
-    CK(dalloc(&h->counters, kCounters));
-    CK(dalloc(&h->block_sums, kScanBlocks + 1));
-    CK(dalloc(&h->acc, 8));
-  }
+  if (!h->counters) CK(dalloc(&h->counters, kCounters));
+  if (!h->block_sums) CK(dalloc(&h->block_sums, kScanBlocks + 1));
+  if (!h->acc) CK(dalloc(&h->acc, 8));
   if (B <= h->bcap) return DD_OK;
   h->scratch_gen++;
-  void* old[] = {h->new_out, h->new_key, h->stat_vis, h->stat_cmps, h->sort_t[0], h->sort_t[1], h->sort_v[0],
-                 h->sort_v[1], h->hist, h->heads, h->flags, h->big, h->gcand, h->gkey,
-                 h->gpos, h->gbits, h->granges};
-  for (void* p : old) dfree(p);
+  // an allocation below may fail: the handle then holds no scratch, and neither
+  // the next build nor dd_destroy meets what was freed here
+  h->bcap = 0;
+  auto drop = [](auto*& p) {
+    dfree(p);
+    p = nullptr;
+  };
+  drop(h->new_out); drop(h->new_key); drop(h->stat_vis); drop(h->stat_cmps);
+  for (int i = 0; i < 2; i++) {
+    drop(h->sort_t[i]);
+    drop(h->sort_v[i]);
+  }
+  drop(h->hist); drop(h->heads); drop(h->flags); drop(h->big); drop(h->gcand);
+  drop(h->gkey); drop(h->gpos); drop(h->gbits); drop(h->granges);
   const uint64_t E = B * h->Rp;
   CK(dalloc(&h->new_out, E));
   CK(dalloc(&h->new_key, E));
