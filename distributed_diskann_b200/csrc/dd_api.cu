@@ -88,10 +88,6 @@ struct dd_index {
   uint64_t qhash_words = 0;
   uint32_t* qev = nullptr;    // evicted lists of the query searches
   uint64_t qev_words = 0;
-  // host calls (search, beam search, prune, ground truth): one device buffer,
-  // kept up to kIoKeepBytes
-  uint8_t* io = nullptr;
-  uint64_t io_bytes = 0;
   bool host_call = false;  // a host call has been staged before
   std::vector<std::pair<uint64_t, LaunchPlan>> qplans;  // query CTA shapes by layout
   // sharded build: the launch shapes and parameters set by dd_shard_begin
@@ -179,13 +175,14 @@ void dfree(void* p) {
   if (p) cudaFree(p);
 }
 
-// The buffers of one host call.  Allocating and freeing device memory in every
-// call cost 70 us (small calls) to several ms (megabytes, and cudaFree waits for
-// the device), and each copy from or to pageable memory 15 us or more: the
-// device buffer stays with the handle, the inputs go up in one copy from a
-// staging buffer and the results come down in one (up to kPinKeepBytes; larger
-// calls copy each array directly).  512 robustPrune tasks 2.4 -> 0.7 ms, one query 450
-// -> 400 us, 30,000 queries of 100 bytes 18 -> 9.6 ms.
+// The buffers of host calls (search, beam search, prune, ground truth).
+// Allocating and freeing device memory in every call cost 70 us (small calls) to
+// several ms (megabytes, and cudaFree waits for the device), and each copy from or
+// to pageable memory 15 us or more: a device buffer is taken from a pool of idle
+// ones, the inputs go up in one copy from a staging buffer and the results come
+// down in one (up to kPinKeepBytes; larger calls copy each array directly).  512
+// robustPrune tasks 2.4 -> 0.7 ms, one query 450 -> 400 us, 30,000 queries of 100
+// bytes 18 -> 9.6 ms.
 constexpr uint64_t kIoKeepBytes = 1ull << 30, kPinKeepBytes = 64ull << 20;
 
 struct IoParts {  // byte offsets, 256-byte aligned
@@ -197,30 +194,24 @@ struct IoParts {  // byte offsets, 256-byte aligned
   }
 };
 
-int ensure_io(dd_index* h, uint64_t bytes) {
-  if (bytes <= h->io_bytes) return DD_OK;
-  dfree(h->io);
-  h->io = nullptr;
-  h->io_bytes = 0;
-  CK(dalloc(&h->io, bytes));
-  h->io_bytes = bytes;
-  return DD_OK;
-}
-
-// Idle pinned buffers, at most kPinKeepBytes of them, for the host calls of all
-// handles; the last handle's end frees them.
-struct PinPool {
+// Idle buffers for the host calls of all handles: pinned ones (kAnyDevice) and
+// those of each device, at most `keep` bytes of either.  The last handle's end
+// frees them, and so does a call that finds no device memory left
+// (with_idle_memory).  A buffer is put back when nothing uses it any more.
+constexpr int kAnyDevice = -1;
+struct BufferPool {
   struct Buf {
     uint8_t* p;
     uint64_t bytes;
+    int device;
   };
   std::mutex mu;
   std::vector<Buf> idle;
   uint64_t handles = 0;
 
-  void drop(size_t i) {
-    cudaFreeHost(idle[i].p);
-    idle.erase(idle.begin() + i);
+  static void release(const Buf& b) {
+    if (b.device == kAnyDevice) cudaFreeHost(b.p);
+    else cudaFree(b.p);
   }
   void open() {
     std::lock_guard<std::mutex> g(mu);
@@ -228,39 +219,102 @@ struct PinPool {
   }
   void close() {
     std::lock_guard<std::mutex> g(mu);
-    if (--handles == 0)
-      while (!idle.empty()) drop(idle.size() - 1);
+    if (--handles) return;
+    for (const Buf& b : idle) release(b);
+    idle.clear();
   }
   // the smallest that fits
-  Buf get(uint64_t bytes) {
+  Buf get(uint64_t bytes, int device) {
     std::lock_guard<std::mutex> g(mu);
     size_t best = idle.size();
     for (size_t i = 0; i < idle.size(); i++)
-      if (idle[i].bytes >= bytes && (best == idle.size() || idle[i].bytes < idle[best].bytes)) best = i;
-    if (best == idle.size()) return {nullptr, 0};
+      if (idle[i].device == device && idle[i].bytes >= bytes &&
+          (best == idle.size() || idle[i].bytes < idle[best].bytes))
+        best = i;
+    if (best == idle.size()) return {nullptr, 0, device};
     const Buf b = idle[best];
     idle.erase(idle.begin() + best);
     return b;
   }
   // beyond the bound the smallest go first: a larger one serves their calls too
-  void put(Buf b) {
+  void put(const Buf& b, uint64_t keep) {
+    if (b.bytes > keep) return release(b);
     std::lock_guard<std::mutex> g(mu);
     idle.push_back(b);
-    uint64_t total = 0;
-    for (const Buf& x : idle) total += x.bytes;
-    while (total > kPinKeepBytes) {
-      size_t s = 0;
-      for (size_t i = 1; i < idle.size(); i++)
-        if (idle[i].bytes < idle[s].bytes) s = i;
-      total -= idle[s].bytes;
-      drop(s);
+    for (;;) {
+      uint64_t total = 0;
+      size_t s = idle.size();
+      for (size_t i = 0; i < idle.size(); i++) {
+        if (idle[i].device != b.device) continue;
+        total += idle[i].bytes;
+        if (s == idle.size() || idle[i].bytes < idle[s].bytes) s = i;
+      }
+      if (total <= keep) return;
+      release(idle[s]);
+      idle.erase(idle.begin() + s);
     }
   }
+  // frees the idle buffers of a device; false: there were none
+  bool drop(int device) {
+    std::lock_guard<std::mutex> g(mu);
+    bool any = false;
+    for (size_t i = idle.size(); i-- > 0;)
+      if (idle[i].device == device) {
+        release(idle[i]);
+        idle.erase(idle.begin() + i);
+        any = true;
+      }
+    return any;
+  }
 };
-PinPool& pin_pool() {
-  static PinPool* pool = new PinPool;  // no destructor: the CUDA runtime may be gone by then
-  return *pool;
+BufferPool& pool() {
+  static BufferPool* p = new BufferPool;  // no destructor: the CUDA runtime may be gone by then
+  return *p;
 }
+
+// Runs a call.  When device memory ran out while the pool held idle buffers of the
+// device, those are freed and the call is run again.
+template <typename F>
+int with_idle_memory(int device, F&& call) {
+  for (;;) {
+    const int rc = call();
+    if (rc != DD_ERR_OOM) return rc;
+    cudaGetLastError();
+    if (!pool().drop(device)) return rc;
+  }
+}
+template <typename F>
+int with_idle_memory(dd_index* h, F&& call) {
+  return with_idle_memory(h ? h->device : 0, call);
+}
+
+// The device buffer of one host call.  It is put back once the handle's stream
+// has run out (an error may leave copies or kernels in flight).
+class DeviceBuffer {
+ public:
+  explicit DeviceBuffer(dd_index* h) : h_(h) {}
+  ~DeviceBuffer() {
+    if (!buf_.p) return;
+    cudaStreamSynchronize(h_->stream);
+    pool().put(buf_, kIoKeepBytes);
+  }
+  DeviceBuffer(const DeviceBuffer&) = delete;
+  DeviceBuffer& operator=(const DeviceBuffer&) = delete;
+  int take(uint64_t bytes) {
+    dd_index* h = h_;
+    buf_ = pool().get(bytes, h->device);
+    if (buf_.p) return DD_OK;
+    uint8_t* p = nullptr;
+    CK(dalloc(&p, bytes));
+    buf_ = {p, bytes, h->device};
+    return DD_OK;
+  }
+  uint8_t* get() const { return buf_.p; }
+
+ private:
+  dd_index* h_;
+  BufferPool::Buf buf_{nullptr, 0, 0};
+};
 
 // Host staging of one call, at least `bytes`; p is null when the call is too
 // large for it.  A handle's first call takes pageable memory (still one copy each
@@ -271,15 +325,15 @@ class Staging {
  public:
   uint8_t* p = nullptr;
 
-  Staging(dd_index* h, uint64_t bytes) : h_(h) {
+  Staging(dd_index* h, uint64_t bytes) {
     if (bytes > kPinKeepBytes) return;
-    buf_ = pin_pool().get(bytes);
+    buf_ = pool().get(bytes, kAnyDevice);
     p = buf_.p;
     if (!p && h->host_call) {
       uint64_t want = 1u << 20;
       while (want < bytes) want *= 2;
       if (cudaHostAlloc((void**)&p, want, cudaHostAllocPortable) == cudaSuccess) {
-        buf_ = {p, want};
+        buf_ = {p, want, kAnyDevice};
       } else {
         cudaGetLastError();
         p = nullptr;
@@ -290,26 +344,18 @@ class Staging {
     }
     h->host_call = true;
   }
+  // (a DeviceBuffer made after it is put back before, which waits for the copies)
   ~Staging() {
-    if (p) cudaStreamSynchronize(h_->stream);  // an error may leave a copy in flight
     std::free(heap_);
-    if (buf_.p) pin_pool().put(buf_);
+    if (buf_.p) pool().put(buf_, kPinKeepBytes);
   }
   Staging(const Staging&) = delete;
   Staging& operator=(const Staging&) = delete;
 
  private:
-  dd_index* h_;
-  PinPool::Buf buf_{nullptr, 0};
+  BufferPool::Buf buf_{nullptr, 0, kAnyDevice};
   uint8_t* heap_ = nullptr;
 };
-
-void release_io(dd_index* h) {
-  if (h->io_bytes <= kIoKeepBytes) return;
-  dfree(h->io);
-  h->io = nullptr;
-  h->io_bytes = 0;
-}
 
 // (a 2-D copy refuses such a stride, stage_rows does not look at it)
 int check_query_stride(dd_index* h, uint64_t qstride) {
@@ -812,8 +858,8 @@ int build_sequence(dd_index* h, const std::vector<std::pair<uint64_t, uint64_t>>
 
 extern "C" {
 
-int dd_create(int dtype, int metric, uint64_t n, uint32_t d, uint32_t R, int device,
-              dd_index** out) {
+static int create(int dtype, int metric, uint64_t n, uint32_t d, uint32_t R, int device,
+                  dd_index** out) {
   dd_index* h = nullptr;
   if (!out) return DD_ERR_ARG;
   *out = nullptr;
@@ -822,7 +868,7 @@ int dd_create(int dtype, int metric, uint64_t n, uint32_t d, uint32_t R, int dev
   if (R > kMaxRp) return DD_ERR_UNSUPPORTED;
   if ((uint64_t)d * esize(dtype) > 1024) return DD_ERR_UNSUPPORTED;
   h = new dd_index();
-  pin_pool().open();
+  pool().open();
   h->dtype = dtype;
   h->metric = metric;
   h->n = n;
@@ -855,6 +901,11 @@ int dd_create(int dtype, int metric, uint64_t n, uint32_t d, uint32_t R, int dev
   return DD_OK;
 }
 
+int dd_create(int dtype, int metric, uint64_t n, uint32_t d, uint32_t R, int device,
+              dd_index** out) {
+  return with_idle_memory(device, [&] { return create(dtype, metric, n, d, R, device, out); });
+}
+
 int dd_destroy(dd_index* h) {
   if (!h) return DD_OK;
   cudaSetDevice(h->device);
@@ -868,14 +919,13 @@ int dd_destroy(dd_index* h) {
   dfree(h->qcls);
   dfree(h->qhash);
   dfree(h->qev);
-  dfree(h->io);
   if (h->gexec) cudaGraphExecDestroy(h->gexec);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   for (cudaStream_t a : h->fork.aux)
     if (a) cudaStreamDestroy(a);
   for (cudaEvent_t e : {h->fork.forked, h->fork.joined[0], h->fork.joined[1]})
     if (e) cudaEventDestroy(e);
-  pin_pool().close();
+  pool().close();
   delete h;
   return DD_OK;
 }
@@ -989,7 +1039,7 @@ int dd_load_points_file(dd_index* h, const char* path) {
   return DD_OK;
 }
 
-int dd_upload_graph(dd_index* h, const uint32_t* rows) {
+static int upload_graph(dd_index* h, const uint32_t* rows) {
   if (!h || !rows) return DD_ERR_ARG;
   CK(cudaSetDevice(h->device));
   uint32_t* tmp = nullptr;
@@ -1005,7 +1055,11 @@ int dd_upload_graph(dd_index* h, const uint32_t* rows) {
   return check_error_word(h);
 }
 
-int dd_download_graph(dd_index* h, uint32_t* rows) {
+int dd_upload_graph(dd_index* h, const uint32_t* rows) {
+  return with_idle_memory(h, [&] { return upload_graph(h, rows); });
+}
+
+static int download_graph(dd_index* h, uint32_t* rows) {
   if (!h || !rows) return DD_ERR_ARG;
   CK(cudaSetDevice(h->device));
   // the reference-layout rows are assembled in a buffer kept by the handle
@@ -1015,6 +1069,10 @@ int dd_download_graph(dd_index* h, uint32_t* rows) {
                      h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return DD_OK;
+}
+
+int dd_download_graph(dd_index* h, uint32_t* rows) {
+  return with_idle_memory(h, [&] { return download_graph(h, rows); });
 }
 
 int dd_save_graph_file(dd_index* h, const char* path) {
@@ -1232,7 +1290,7 @@ int build_once(dd_index* h, const dd_build_params* P, uint32_t vcap, dd_stats* s
 
 extern "C" {
 
-int dd_build(dd_index* h, const dd_build_params* P, dd_stats* stats) {
+static int build(dd_index* h, const dd_build_params* P, dd_stats* stats) {
   if (!h || !P) return DD_ERR_ARG;
   if (P->L == 0 || P->L > kMaxL) return fail(h, DD_ERR_UNSUPPORTED, "L must be in [1, %u]", kMaxL);
   uint32_t start = P->knn_mode ? 0 : P->start_point;  // include/index.h:127
@@ -1261,6 +1319,10 @@ int dd_build(dd_index* h, const dd_build_params* P, dd_stats* stats) {
     }
     return rc;
   }
+}
+
+int dd_build(dd_index* h, const dd_build_params* P, dd_stats* stats) {
+  return with_idle_memory(h, [&] { return build(h, P, stats); });
 }
 
 // ---------------------------------------------------------------- sharded build
@@ -1309,7 +1371,7 @@ RoundArgs shard_round_args(dd_index* h, uint64_t floor, uint64_t B, uint32_t* ro
 }
 }  // namespace
 
-int dd_shard_begin(dd_index* h, const dd_build_params* P, uint64_t max_batch) {
+static int shard_begin(dd_index* h, const dd_build_params* P, uint64_t max_batch) {
   if (!h || !P) return DD_ERR_ARG;
   if (P->L == 0 || P->L > kMaxL) return fail(h, DD_ERR_UNSUPPORTED, "L must be in [1, %u]", kMaxL);
   if (P->two_pass || P->knn_mode)
@@ -1341,6 +1403,10 @@ int dd_shard_begin(dd_index* h, const dd_build_params* P, uint64_t max_batch) {
   CK(cudaStreamSynchronize(h->stream));
   h->shard_ready = true;
   return DD_OK;
+}
+
+int dd_shard_begin(dd_index* h, const dd_build_params* P, uint64_t max_batch) {
+  return with_idle_memory(h, [&] { return shard_begin(h, P, max_batch); });
 }
 
 int dd_shard_search_prune(dd_index* h, uint64_t lo, uint64_t hi, uint32_t* rows) {
@@ -1619,14 +1685,17 @@ int dd_search_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
                      const uint32_t* L_per_query, uint32_t Lmax, uint32_t k, double cut,
                      uint64_t limit, uint32_t degree_limit, uint32_t start, int skip_self,
                      uint32_t* ids, float* dists, uint32_t* visited, uint32_t* cmps) {
-  return search_on_device(h, queries, nq, qstride, L_per_query, Lmax, k, cut, limit, degree_limit,
-                          start, skip_self, ids, dists, visited, cmps, kAllQueryClasses);
+  return with_idle_memory(h, [&] {
+    return search_on_device(h, queries, nq, qstride, L_per_query, Lmax, k, cut, limit,
+                            degree_limit, start, skip_self, ids, dists, visited, cmps,
+                            kAllQueryClasses);
+  });
 }
 
-int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
-              const uint32_t* L_per_query, uint32_t k, double cut, uint64_t limit,
-              uint32_t degree_limit, uint32_t start, int skip_self, uint32_t* ids, float* dists,
-              uint32_t* visited, uint32_t* cmps) {
+static int search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
+                  const uint32_t* L_per_query, uint32_t k, double cut, uint64_t limit,
+                  uint32_t degree_limit, uint32_t start, int skip_self, uint32_t* ids, float* dists,
+                  uint32_t* visited, uint32_t* cmps) {
   if (!h || !queries || !L_per_query || !ids || !dists) return DD_ERR_ARG;
   if (nq == 0) return DD_OK;
   int rc = check_query_stride(h, qstride);
@@ -1643,11 +1712,12 @@ int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
   const uint64_t o_q = io.take(nq * ds), o_L = io.take(nq * 4), in_bytes = io.total;
   const uint64_t o_i = io.take(nq * k * 4ull), o_d = io.take(nq * k * 4ull), o_v = io.take(nq * 4),
                  o_c = io.take(nq * 4), out_bytes = io.total - in_bytes;
-  rc = ensure_io(h, io.total);
-  if (rc) return rc;
-  uint8_t* dev = h->io;
   const Staging staged(h, std::max(in_bytes, out_bytes));
   uint8_t* const pin = staged.p;
+  DeviceBuffer buf(h);
+  rc = buf.take(io.total);
+  if (rc) return rc;
+  uint8_t* dev = buf.get();
   if (pin) {
     stage_rows(pin + o_q, ds, (const uint8_t*)queries, qstride, rb, nq);
     std::memcpy(pin + o_L, L_per_query, nq * 4);
@@ -1679,17 +1749,25 @@ int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) rc = check_error_word(h);
   }
-  if (rc || e != cudaSuccess) cudaStreamSynchronize(h->stream);  // the buffers are free again
-  release_io(h);
   CK(e);
   return rc;
 }
 
-int dd_beam_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
-                   const int64_t* self_ids, uint32_t L, uint32_t k, double cut, uint64_t limit,
-                   uint32_t degree_limit, uint32_t start, uint32_t vcap, uint32_t* fr_ids,
-                   float* fr_dists, uint32_t* fr_sizes, uint32_t* vis_ids, float* vis_dists,
-                   uint32_t* vis_sizes, uint32_t* cmps) {
+int dd_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
+              const uint32_t* L_per_query, uint32_t k, double cut, uint64_t limit,
+              uint32_t degree_limit, uint32_t start, int skip_self, uint32_t* ids, float* dists,
+              uint32_t* visited, uint32_t* cmps) {
+  return with_idle_memory(h, [&] {
+    return search(h, queries, nq, qstride, L_per_query, k, cut, limit, degree_limit, start,
+                  skip_self, ids, dists, visited, cmps);
+  });
+}
+
+static int beam_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
+                       const int64_t* self_ids, uint32_t L, uint32_t k, double cut, uint64_t limit,
+                       uint32_t degree_limit, uint32_t start, uint32_t vcap, uint32_t* fr_ids,
+                       float* fr_dists, uint32_t* fr_sizes, uint32_t* vis_ids, float* vis_dists,
+                       uint32_t* vis_sizes, uint32_t* cmps) {
   if (!h || !queries || !self_ids || nq == 0) return DD_ERR_ARG;
   if (L == 0 || L > kMaxL) return fail(h, DD_ERR_UNSUPPORTED, "L must be in [1, %u]", kMaxL);
   if (start >= h->n) return fail(h, DD_ERR_ARG, "start point >= n");
@@ -1703,9 +1781,10 @@ int dd_beam_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
                  o_fd = io.take(nq * L * 4ull), o_fn = io.take(nq * 4),
                  o_vi = io.take(nq * vcap * 4ull), o_vd = io.take(nq * vcap * 4ull),
                  o_vn = io.take(nq * 4), o_cm = io.take(nq * 4);
-  int rc = ensure_io(h, io.total);
+  DeviceBuffer buf(h);
+  int rc = buf.take(io.total);
   if (rc) return rc;
-  uint8_t* dev = h->io;
+  uint8_t* dev = buf.get();
   uint8_t* dq = dev + o_q;
   int64_t* dself = (int64_t*)(dev + o_s);
   uint32_t *dfi = (uint32_t*)(dev + o_fi), *dfn = (uint32_t*)(dev + o_fn),
@@ -1735,15 +1814,24 @@ int dd_beam_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   if (e == cudaSuccess) e = cudaMemcpyAsync(vis_sizes, dvn, nq * 4, cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(cmps, dcm, nq * 4, cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (e != cudaSuccess) cudaStreamSynchronize(h->stream);
-  release_io(h);
   CK(e);
   return check_error_word(h);
 }
 
-int dd_robust_prune(dd_index* h, uint32_t ntasks, const uint32_t* p, const uint64_t* offsets,
-                    const uint32_t* cand_ids, const float* cand_dists, double alpha,
-                    uint32_t* out, uint32_t* out_len) {
+int dd_beam_search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
+                   const int64_t* self_ids, uint32_t L, uint32_t k, double cut, uint64_t limit,
+                   uint32_t degree_limit, uint32_t start, uint32_t vcap, uint32_t* fr_ids,
+                   float* fr_dists, uint32_t* fr_sizes, uint32_t* vis_ids, float* vis_dists,
+                   uint32_t* vis_sizes, uint32_t* cmps) {
+  return with_idle_memory(h, [&] {
+    return beam_search(h, queries, nq, qstride, self_ids, L, k, cut, limit, degree_limit, start,
+                       vcap, fr_ids, fr_dists, fr_sizes, vis_ids, vis_dists, vis_sizes, cmps);
+  });
+}
+
+static int robust_prune(dd_index* h, uint32_t ntasks, const uint32_t* p, const uint64_t* offsets,
+                        const uint32_t* cand_ids, const float* cand_dists, double alpha,
+                        uint32_t* out, uint32_t* out_len) {
   if (!h || !p || !offsets || !out || !out_len) return DD_ERR_ARG;
   if (ntasks == 0) return DD_OK;
   for (uint32_t t = 0; t < ntasks; t++)
@@ -1764,11 +1852,13 @@ int dd_robust_prune(dd_index* h, uint32_t ntasks, const uint32_t* p, const uint6
   const bool global = !(alpha > 1e-3 && alpha < 1e3) || !prune_tasks_in_shared(view(h), most);
   const uint64_t o_gc = io.take(global ? ws * 4 : 0), o_gk = io.take(global ? ws * 4 : 0),
                  o_gl = io.take(global ? (3 * ws + (uint64_t)ntasks * kGlobalStackInts) * 4 : 0);
-  int rc = ensure_io(h, io.total);
-  if (rc) return rc;
-  uint8_t* dev = h->io;
   const Staging staged(h, std::max(in_bytes, out_bytes));
   uint8_t* const pin = staged.p;
+  std::vector<uint32_t> heap(pin ? 0 : (uint64_t)ntasks * h->Rp);
+  DeviceBuffer buf(h);
+  int rc = buf.take(io.total);
+  if (rc) return rc;
+  uint8_t* dev = buf.get();
   cudaError_t e = cudaSuccess;
   if (pin) {
     std::memcpy(pin + o_off, offsets, (ntasks + 1) * 8ull);
@@ -1792,22 +1882,27 @@ int dd_robust_prune(dd_index* h, uint32_t ntasks, const uint32_t* p, const uint6
     else launch_prune_tasks_shared(view(h), pa, most, h->stream);
     e = cudaGetLastError();
   }
-  std::vector<uint32_t> heap(pin ? 0 : (uint64_t)ntasks * h->Rp);
   const uint32_t* o = pin ? (const uint32_t*)pin : heap.data();
   if (e == cudaSuccess)
     e = cudaMemcpyAsync((void*)o, dev + o_out, (uint64_t)ntasks * h->Rp * 4, cudaMemcpyDeviceToHost,
                         h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  else cudaStreamSynchronize(h->stream);
-  release_io(h);
   CK(e);
   for (uint32_t t = 0; t < ntasks; t++) {
-    uint32_t len = 0;
-    while (len < h->R && o[(uint64_t)t * h->Rp + len] != DD_NONE) len++;
-    out_len[t] = len;
-    for (uint32_t j = 0; j < h->R; j++) out[(uint64_t)t * h->R + j] = j < len ? o[(uint64_t)t * h->Rp + j] : 0u;
+    const uint32_t *row = o + (uint64_t)t * h->Rp, *end = row + h->R;
+    const uint64_t len = std::find(row, end, DD_NONE) - row;
+    out_len[t] = (uint32_t)len;
+    std::fill(std::copy(row, row + len, out + (uint64_t)t * h->R), out + (uint64_t)(t + 1) * h->R, 0u);
   }
   return check_error_word(h);
+}
+
+int dd_robust_prune(dd_index* h, uint32_t ntasks, const uint32_t* p, const uint64_t* offsets,
+                    const uint32_t* cand_ids, const float* cand_dists, double alpha,
+                    uint32_t* out, uint32_t* out_len) {
+  return with_idle_memory(h, [&] {
+    return robust_prune(h, ntasks, p, offsets, cand_ids, cand_dists, alpha, out, out_len);
+  });
 }
 
 // one launch of the ground truth: nq queries, arguments checked
@@ -1818,14 +1913,15 @@ static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint
   IoParts io;
   const uint64_t o_q = io.take(nq * ds), o_i = io.take(nq * k * 4ull), o_d = io.take(nq * k * 4ull),
                  o_w = io.take(1024 + groundtruth_work_bytes(ix, nq, k, h->sm_count));
-  int rc = ensure_io(h, io.total);
-  if (rc) return rc;
-  uint8_t* dq = h->io + o_q;
-  uint32_t* di = (uint32_t*)(h->io + o_i);
-  float* dd = (float*)(h->io + o_d);
-  uint8_t* work = h->io + ((o_w + 1023) & ~(uint64_t)1023);
   const Staging staged(h, std::max<uint64_t>(nq * ds, nq * k * 8ull + 64));
   uint8_t* const pin = staged.p;
+  DeviceBuffer buf(h);
+  int rc = buf.take(io.total);
+  if (rc) return rc;
+  uint8_t* dq = buf.get() + o_q;
+  uint32_t* di = (uint32_t*)(buf.get() + o_i);
+  float* dd = (float*)(buf.get() + o_d);
+  uint8_t* work = buf.get() + ((o_w + 1023) & ~(uint64_t)1023);
   uint8_t* parts = nullptr;
   uint32_t *over = nullptr, left[2] = {0, 0};  // queries left, error bits
   bool ok = true;
@@ -1875,7 +1971,6 @@ static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint
   }
   if (!ok || e != cudaSuccess) cudaStreamSynchronize(h->stream);
   dfree(parts);
-  release_io(h);
   CK(e);
   if (!ok) return fail(h, DD_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   return device_error(h, left[1]);
@@ -1895,8 +1990,10 @@ int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   while (batch > 4096 && groundtruth_work_bytes(ix, batch, k, h->sm_count) > (2ull << 30))
     batch = (batch + 1) / 2;
   for (uint64_t q = 0; q < nq; q += batch) {
-    const int rc = groundtruth_batch(h, (const uint8_t*)queries + q * qstride, std::min(batch, nq - q),
-                                     qstride, k, ids + q * k, dists + q * k);
+    const int rc = with_idle_memory(h, [&] {
+      return groundtruth_batch(h, (const uint8_t*)queries + q * qstride, std::min(batch, nq - q),
+                               qstride, k, ids + q * k, dists + q * k);
+    });
     if (rc) return rc;
   }
   return DD_OK;

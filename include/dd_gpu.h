@@ -111,6 +111,10 @@ typedef struct dd_stats {
 int dd_create(int dtype, int metric, uint64_t n, uint32_t d, uint32_t R, int device,
               dd_index** out);
 int dd_destroy(dd_index* h);
+/* Calls with host arrays keep their buffers for the next such call of any handle:
+ * at most 1 GB of device memory per device and 64 MB of pinned host memory lie
+ * idle.  They are freed by the last handle's dd_destroy, and the device memory by
+ * any call that finds none left. */
 const char* dd_last_error(const dd_index* h);
 /* all work of the handle is issued on this CUDA stream (cudaStream_t); 0 = default */
 int dd_set_stream(dd_index* h, void* stream);

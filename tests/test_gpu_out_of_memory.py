@@ -1,4 +1,5 @@
-"""Calls that run out of device memory fail with an error and leave the handle usable."""
+"""Calls that run out of device memory fail with an error and leave the handle usable, but
+not before the idle buffers of earlier host calls are given back."""
 import contextlib
 
 import numpy as np
@@ -68,3 +69,41 @@ def test_a_build_that_runs_out_of_memory_leaves_the_handle_usable():
         gi.build(64, 1.2)  # its scratch is there
     np.testing.assert_array_equal(_rows(gi), large)
     gi.close()
+
+
+def test_idle_buffers_of_host_calls_are_given_back():
+    """A float ground truth leaves a buffer of 300 MB; calls of the same handle and of
+    others then find less free memory than they need."""
+    import torch
+
+    n, d = 300_000, 256
+    base = torch.randn(n, d, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    q = base[:40].cpu().numpy()
+    gi = GpuIndex(np.float32, "l2", n, d, 64)
+    gi.upload_points(base)
+    torch.cuda.synchronize()
+    del base
+    small = D.gen_mixture_f32(200_000, 64, 60, 3)
+
+    def ground_truth():
+        ids, _ = gi.groundtruth(q, 3)
+        np.testing.assert_array_equal(ids[:, 0], np.arange(40))
+
+    ground_truth()
+    with free_memory(40):
+        g = gi.graph()  # 78 MB of rows
+    assert not g.any()
+    ground_truth()
+    with free_memory(40):
+        other = GpuIndex(small.dtype, "l2", 200_000, 64, 64)  # 102 MB
+        other.upload_points(small)
+    ground_truth()
+    with free_memory(60):
+        other.build(64, 1.2, max_build=20_000)  # 100 MB of scratch
+        ids = other.search(small[:50], 1, 20, skip_self=False)[0]
+    want = GpuIndex(small.dtype, "l2", 200_000, 64, 64)
+    want.upload_points(small)
+    want.build(64, 1.2, max_build=20_000)
+    np.testing.assert_array_equal(ids, want.search(small[:50], 1, 20, skip_self=False)[0])
+    for x in (gi, other, want):
+        x.close()
