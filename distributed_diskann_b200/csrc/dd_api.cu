@@ -1905,14 +1905,16 @@ int dd_robust_prune(dd_index* h, uint32_t ntasks, const uint32_t* p, const uint6
   });
 }
 
+constexpr uint64_t kGtMinSlab = 8192;
+
 // one launch of the ground truth: nq queries, arguments checked
 static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride,
-                             uint32_t k, uint32_t* ids, float* dists) {
+                             uint32_t k, const GtLimits& lim, uint32_t* ids, float* dists) {
   uint64_t rb = (uint64_t)h->d * esize(h->dtype), ds = h->stride;
   const IndexView ix = view(h);
   IoParts io;
   const uint64_t o_q = io.take(nq * ds), o_i = io.take(nq * k * 4ull), o_d = io.take(nq * k * 4ull),
-                 o_w = io.take(1024 + groundtruth_work_bytes(ix, nq, k, h->sm_count));
+                 o_w = io.take(1024 + groundtruth_work_bytes(ix, nq, k, lim));
   const Staging staged(h, std::max<uint64_t>(nq * ds, nq * k * 8ull + 64));
   uint8_t* const pin = staged.p;
   DeviceBuffer buf(h);
@@ -1935,7 +1937,7 @@ static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint
       e = cudaMemcpy2DAsync(dq, ds, queries, qstride, rb, nq, cudaMemcpyHostToDevice, h->stream);
   }
   if (e == cudaSuccess) {
-    ok = launch_groundtruth(ix, dq, ds, nq, k, di, dd, work, h->sm_count, h->stream, &over);
+    ok = launch_groundtruth(ix, dq, ds, nq, k, di, dd, work, lim, h->stream, &over);
     e = cudaGetLastError();
   }
   if (ok) {
@@ -1959,11 +1961,14 @@ static int groundtruth_batch(dd_index* h, const void* queries, uint64_t nq, uint
     if (const uint32_t todo = e == cudaSuccess ? left[0] : 0u) {
       // float queries whose candidates the screen could not bound
       const uint64_t per = (uint64_t)groundtruth_exact_chunks(ix) * k * 12;
-      const uint32_t batch = (uint32_t)std::min<uint64_t>(todo, std::max<uint64_t>(1, (256ull << 20) / per));
-      e = dalloc(&parts, batch * per);
+      uint32_t batch = (uint32_t)std::min<uint64_t>(todo, std::max<uint64_t>(1, (256ull << 20) / per));
+      while ((e = dalloc(&parts, batch * per)) == cudaErrorMemoryAllocation && batch > 1) {
+        cudaGetLastError();
+        batch = (batch + 1) / 2;
+      }
       for (uint32_t f = 0; e == cudaSuccess && f < todo; f += batch) {
         launch_groundtruth_exact(ix, dq, ds, nq, f, std::min(batch, todo - f), k, di, dd, work,
-                                 h->sm_count, parts, h->stream);
+                                 lim, parts, h->stream);
         e = cudaGetLastError();
       }
       if (e == cudaSuccess) download();
@@ -1987,14 +1992,34 @@ int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   // workspace within 2 GB, but at least 4096 (a float base is converted once a batch)
   const IndexView ix = view(h);
   uint64_t batch = nq;
-  while (batch > 4096 && groundtruth_work_bytes(ix, batch, k, h->sm_count) > (2ull << 30))
-    batch = (batch + 1) / 2;
-  for (uint64_t q = 0; q < nq; q += batch) {
+  GtLimits lim{h->sm_count};
+  auto bytes = [&] { return groundtruth_work_bytes(ix, batch, k, lim); };
+  while (batch > 4096 && bytes() > (2ull << 30)) batch = (batch + 1) / 2;
+  // Where the device has less room than that, and for tests with a bound set by
+  // DD_GT_WORK_BYTES: fewer queries at a time, then smaller slabs and fewer CTAs,
+  // down to some 40 MB for a base of a million rows.
+  auto shrink = [&] {
+    if (batch > 256) {
+      batch = (batch + 1) / 2;
+      return true;
+    }
+    if (lim.grid == 1 && lim.slab == kGtMinSlab) return false;
+    lim.grid = (lim.grid + 1) / 2;
+    lim.slab = std::max<uint64_t>(kGtMinSlab, lim.slab / 2);
+    return true;
+  };
+  if (const char* e = getenv("DD_GT_WORK_BYTES")) {
+    const uint64_t bound = strtoull(e, nullptr, 10);
+    while (bytes() > bound && shrink()) {}
+  }
+  for (uint64_t q = 0; q < nq;) {
+    const uint64_t m = std::min(batch, nq - q);
     const int rc = with_idle_memory(h, [&] {
-      return groundtruth_batch(h, (const uint8_t*)queries + q * qstride, std::min(batch, nq - q),
-                               qstride, k, ids + q * k, dists + q * k);
+      return groundtruth_batch(h, (const uint8_t*)queries + q * qstride, m, qstride, k, lim,
+                               ids + q * k, dists + q * k);
     });
-    if (rc) return rc;
+    if (rc == DD_OK) q += m;
+    else if (rc != DD_ERR_OOM || !shrink()) return rc;
   }
   return DD_OK;
 }

@@ -158,7 +158,6 @@ constexpr uint32_t kGtTileBytes = kGtTile * kGtBlockBytes;
 // compacted one in most steps, and the step's TMEM buffer waited for it: 4.3 ms
 // instead of 3.7 ms for the uint8 call below.)
 constexpr uint32_t kGtCap = 128;
-constexpr uint64_t kGtSlab = 1u << 20; // float base rows converted at a time
 // |p|^2 of the rows past n, and the scores that no point lies below and no such
 // row reaches (integer rows of 1024 bytes: scores above -2^27)
 constexpr int kGtIntPad = 1 << 30, kGtIntNone = -(1 << 29);
@@ -187,7 +186,7 @@ struct GtShape {
 // 1.48 ms without the sample); one of fewer than k tiles is not.
 constexpr uint32_t kGtGroups = 128, kGtSampleOf = 5;
 
-static GtShape gt_shape(const IndexView& ix, uint64_t nq, uint32_t k, int sm_count) {
+static GtShape gt_shape(const IndexView& ix, uint64_t nq, uint32_t k, const GtLimits& lim) {
   GtShape s{};
   s.f32 = ix.dtype == DD_F32;
   s.dp = (ix.d + 15) & ~15u;
@@ -202,12 +201,12 @@ static GtShape gt_shape(const IndexView& ix, uint64_t nq, uint32_t k, int sm_cou
   const uint32_t fixed = s.mtiles * s.nkb * kGtTileBytes + s.rows * 16;
   s.stages = std::min<uint32_t>(8, (226 * 1024 - fixed) / kGtTileBytes);
   s.smem = fixed + s.stages * kGtTileBytes;
-  s.slab = s.f32 ? std::min<uint64_t>(ix.n, kGtSlab) : ix.n;
+  s.slab = s.f32 ? std::min<uint64_t>(ix.n, lim.slab) : ix.n;
   s.nslabs = (ix.n + s.slab - 1) / s.slab;
   s.qtiles = (nq + s.rows - 1) / s.rows;
   s.btiles = (s.slab + kGtTile - 1) / kGtTile;
   const uint64_t total = s.qtiles * s.btiles;
-  s.grid = std::min<uint64_t>(sm_count, total);
+  s.grid = std::min<uint64_t>(lim.grid, total);
   s.per = (total + s.grid - 1) / s.grid;
   s.segs = (s.btiles - 1) / s.per + 2;
   s.groups = s.btiles >= k ? std::min<uint64_t>(kGtGroups, s.btiles) : 0;
@@ -250,8 +249,8 @@ static GtWork gt_work(const IndexView& ix, uint64_t nq, const GtShape& s) {
   return w;
 }
 
-uint64_t groundtruth_work_bytes(const IndexView& ix, uint64_t nq, uint32_t k, int sm_count) {
-  return gt_work(ix, nq, gt_shape(ix, nq, k, sm_count)).total;
+uint64_t groundtruth_work_bytes(const IndexView& ix, uint64_t nq, uint32_t k, const GtLimits& lim) {
+  return gt_work(ix, nq, gt_shape(ix, nq, k, lim)).total;
 }
 
 // ============================================================ preparation
@@ -968,13 +967,13 @@ static bool gt_tensor_map(CUtensorMap* m, bool f32, const void* p, uint64_t row_
 
 template <bool F32, int MT, int MTILES>
 static void gt_launch(const GtShape& s, const CUtensorMap& qm, const CUtensorMap& bm, GtArgs g,
-                      uint32_t* thr0, int sm_count, cudaStream_t st) {
+                      uint32_t* thr0, int max_grid, cudaStream_t st) {
   if (s.groups && g.id0 == 0) {  // the first slab's sample serves all slabs
     GtArgs a = g;
     a.gtiles = (uint32_t)s.gtiles;
     a.btiles = (uint32_t)(s.groups * s.gtiles);
     a.gstride = (uint32_t)(s.btiles / a.btiles);
-    const uint64_t total = s.qtiles * a.btiles, grid = std::min<uint64_t>(sm_count, total);
+    const uint64_t total = s.qtiles * a.btiles, grid = std::min<uint64_t>(max_grid, total);
     a.per = (uint32_t)((total + grid - 1) / grid);
     set_smem(k_gt_tc<F32, MT, MTILES, true>, s.smem);
     k_gt_tc<F32, MT, MTILES, true><<<(unsigned)grid, MTILES * 128 + 64, s.smem, st>>>(qm, bm, a);
@@ -991,9 +990,9 @@ static void gt_launch(const GtShape& s, const CUtensorMap& qm, const CUtensorMap
 // many queries launch_groundtruth_exact must still compute; (*over)[1]: the
 // error bits of these launches (the index's word keeps what other calls left).
 bool launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qstride, uint64_t nq,
-                        uint32_t k, uint32_t* ids, float* dists, uint8_t* work, int sm_count,
+                        uint32_t k, uint32_t* ids, float* dists, uint8_t* work, const GtLimits& lim,
                         cudaStream_t st, uint32_t** over) {
-  const GtShape s = gt_shape(ix, nq, k, sm_count);
+  const GtShape s = gt_shape(ix, nq, k, lim);
   const GtWork w = gt_work(ix, nq, s);
   const bool l2 = ix.metric == DD_L2;
   cudaMemsetAsync(work + w.zero0, 0, w.zero1 - w.zero0, st);
@@ -1058,8 +1057,8 @@ bool launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qs
       k_gt_prep<DD_F32><<<bgrid, 256, 0, st>>>(pts, ix.stride, rows, npad, ix.d, s.dp, l2, true,
                                                work + w.pnorm, scal, bhalf);
       if (!gt_tensor_map(&bm, true, bhalf, 2 * s.dp, rows, 4ull * s.dp)) return false;
-      if (l2) gt_launch<true, DD_L2, 1>(s, qm, bm, g, thr0, sm_count, st);
-      else gt_launch<true, DD_MIPS, 1>(s, qm, bm, g, thr0, sm_count, st);
+      if (l2) gt_launch<true, DD_L2, 1>(s, qm, bm, g, thr0, lim.grid, st);
+      else gt_launch<true, DD_MIPS, 1>(s, qm, bm, g, thr0, lim.grid, st);
     } else {
       if (ix.dtype == DD_I8)
         k_gt_prep<DD_I8><<<bgrid, 256, 0, st>>>(pts, ix.stride, rows, npad, ix.d, 0, l2, true,
@@ -1069,11 +1068,11 @@ bool launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qs
                                                 work + w.pnorm, nullptr, nullptr);
       if (!gt_tensor_map(&bm, false, pts, ix.stride, rows, ix.stride)) return false;
       if (s.mtiles == 2) {
-        if (l2) gt_launch<false, DD_L2, 2>(s, qm, bm, g, thr0, sm_count, st);
-        else gt_launch<false, DD_MIPS, 2>(s, qm, bm, g, thr0, sm_count, st);
+        if (l2) gt_launch<false, DD_L2, 2>(s, qm, bm, g, thr0, lim.grid, st);
+        else gt_launch<false, DD_MIPS, 2>(s, qm, bm, g, thr0, lim.grid, st);
       } else {
-        if (l2) gt_launch<false, DD_L2, 1>(s, qm, bm, g, thr0, sm_count, st);
-        else gt_launch<false, DD_MIPS, 1>(s, qm, bm, g, thr0, sm_count, st);
+        if (l2) gt_launch<false, DD_L2, 1>(s, qm, bm, g, thr0, lim.grid, st);
+        else gt_launch<false, DD_MIPS, 1>(s, qm, bm, g, thr0, lim.grid, st);
       }
     }
   }
@@ -1099,9 +1098,9 @@ uint32_t groundtruth_exact_chunks(const IndexView& ix) {
 // from entry `first`; parts: count x chunks x k doubles, then as many ids
 void launch_groundtruth_exact(const IndexView& ix, const uint8_t* queries, uint64_t qstride,
                               uint64_t nq, uint32_t first, uint32_t count, uint32_t k,
-                              uint32_t* ids, float* dists, const uint8_t* work, int sm_count,
-                              uint8_t* parts, cudaStream_t st) {
-  const GtWork w = gt_work(ix, nq, gt_shape(ix, nq, k, sm_count));
+                              uint32_t* ids, float* dists, const uint8_t* work,
+                              const GtLimits& lim, uint8_t* parts, cudaStream_t st) {
+  const GtWork w = gt_work(ix, nq, gt_shape(ix, nq, k, lim));
   const uint32_t* list = (const uint32_t*)(work + w.over_list) + first;
   const uint32_t nchunks = groundtruth_exact_chunks(ix);
   double* pd = (double*)parts;

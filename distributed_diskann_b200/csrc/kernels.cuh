@@ -255,20 +255,28 @@ bool prune_tasks_in_shared(const IndexView& ix, uint64_t most);
 void launch_prune_tasks_shared(const IndexView& ix, const PruneArgs& pa, uint64_t most,
                                cudaStream_t st);
 
+// What the workspace of few queries grows with: each of `grid` CTAs has 128 KB of
+// candidate lists or more per slab, and a slab's rows are kept as BF16 halves
+// (float data).  dd_groundtruth lowers both where memory is short.
+struct GtLimits {
+  int grid;
+  uint64_t slab = 1u << 20;  // float base rows converted at a time
+};
+
 // brute-force ground truth (k_gt.cu): device queries of stride qstride (a
 // multiple of 64, zero padded), a workspace of groundtruth_work_bytes; *over
 // names two device words: how many float queries launch_groundtruth_exact must
 // still compute, and the error bits of the launches.  False: no tensor map
 // could be made.
-uint64_t groundtruth_work_bytes(const IndexView& ix, uint64_t nq, uint32_t k, int sm_count);
+uint64_t groundtruth_work_bytes(const IndexView& ix, uint64_t nq, uint32_t k, const GtLimits& lim);
 bool launch_groundtruth(const IndexView& ix, const uint8_t* queries, uint64_t qstride, uint64_t nq,
-                        uint32_t k, uint32_t* ids, float* dists, uint8_t* work, int sm_count,
+                        uint32_t k, uint32_t* ids, float* dists, uint8_t* work, const GtLimits& lim,
                         cudaStream_t st, uint32_t** over);
 uint32_t groundtruth_exact_chunks(const IndexView& ix);
 void launch_groundtruth_exact(const IndexView& ix, const uint8_t* queries, uint64_t qstride,
                               uint64_t nq, uint32_t first, uint32_t count, uint32_t k,
-                              uint32_t* ids, float* dists, const uint8_t* work, int sm_count,
-                              uint8_t* parts, cudaStream_t st);
+                              uint32_t* ids, float* dists, const uint8_t* work,
+                              const GtLimits& lim, uint8_t* parts, cudaStream_t st);
 
 // sharded build exchange: the rows of the targets this rank's reverse step
 // changed (segments of the grouped pairs, st/heads/counters as in

@@ -240,7 +240,10 @@ int dd_robust_prune_noalloc(dd_index* h, uint32_t ntasks, const uint32_t* p,
                             uint32_t* out, int synchronize);
 
 /* brute-force k nearest neighbours (k <= 32): FP64 distances for float data,
- * exact integers for integer data; ties ordered by id */
+ * exact integers for integer data; ties ordered by id.  The workspace is up to
+ * 2 GB, and for float data 4 bytes x padded d for each of up to 2^20 base rows;
+ * with less device memory free (or a bound set by DD_GT_WORK_BYTES) the call
+ * takes fewer queries and rows at a time, down to some tens of MB */
 int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstride, uint32_t k,
                    uint32_t* ids, float* dists);
 

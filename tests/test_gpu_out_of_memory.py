@@ -107,3 +107,57 @@ def test_idle_buffers_of_host_calls_are_given_back():
     np.testing.assert_array_equal(ids, want.search(small[:50], 1, 20, skip_self=False)[0])
     for x in (gi, other, want):
         x.close()
+
+
+@pytest.mark.parametrize("work_mb", [400, 40, 8, 0])
+@pytest.mark.parametrize("kind", ["u8", "i8", "f32", "ties", "mips"])
+def test_ground_truth_of_a_bounded_workspace(oracle_mod, monkeypatch, kind, work_mb):
+    """Batches of queries (float ones with queries left to the FP64 form on both sides of
+    each boundary), slabs of 8192 rows and up, one CTA and more."""
+    rng = np.random.default_rng(5)
+    n, nq, d = 20_001, 1_300, 24
+    metric = "mips" if kind == "mips" else "l2"
+    if kind in ("u8", "i8"):
+        t, lo = (np.uint8, 0) if kind == "u8" else (np.int8, -128)
+        base = rng.integers(lo, lo + 256, (n, d)).astype(t)
+        q = rng.integers(lo, lo + 256, (nq, d)).astype(t)
+    else:
+        base = rng.standard_normal((n, d), dtype=np.float32)
+        q = rng.standard_normal((nq, d), dtype=np.float32)
+        if kind == "ties":  # hundreds of points at one distance of every third query
+            base = rng.integers(0, 3, (n, d)).astype(np.float32)
+            q[::3] = rng.integers(0, 3, (len(q[::3]), d))
+    monkeypatch.setenv("DD_GT_WORK_BYTES", str(work_mb * MB))
+    gi = GpuIndex(base.dtype, metric, n, d, 8)
+    gi.upload_points(base)
+    for k in (32, 3):
+        ids, ds = gi.groundtruth(q, k)
+        oi, od = oracle_mod.groundtruth(base, q, k, metric=metric)
+        np.testing.assert_array_equal(ids, oi)
+        np.testing.assert_array_equal(ds, od)
+    gi.close()
+
+
+@pytest.mark.parametrize("dtype,nq", [("f32", 300), ("u8", 3_000)])
+def test_ground_truth_with_little_memory_left(dtype, nq):
+    """A workspace of 310 MB (float rows as BF16 halves) or 60 MB (candidate lists) does
+    not fit; a smaller one gives the same answer."""
+    import torch
+
+    n, d = 300_000, 256
+    g = torch.Generator("cuda").manual_seed(2)
+    if dtype == "f32":
+        base = torch.randn(n, d, device="cuda", generator=g)
+    else:
+        base = torch.randint(0, 256, (n, d), device="cuda", generator=g, dtype=torch.uint8)
+    q = base[:nq].cpu().numpy()
+    gi = GpuIndex(np.dtype(np.float32 if dtype == "f32" else np.uint8), "l2", n, d, 8)
+    gi.upload_points(base)
+    torch.cuda.synchronize()
+    del base
+    with free_memory(100 if dtype == "f32" else 24):
+        ids, ds = gi.groundtruth(q, 10)
+    wi, wd = gi.groundtruth(q, 10)
+    np.testing.assert_array_equal(ids, wi)
+    np.testing.assert_array_equal(ds, wd)
+    gi.close()
