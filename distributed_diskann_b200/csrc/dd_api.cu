@@ -273,15 +273,17 @@ BufferPool& pool() {
 }
 
 // Runs a call.  When device memory ran out while the pool held idle buffers of the
-// device, those are freed and the call is run again.
+// device, those are freed and the call is run again: once, since a call that
+// fails late puts its own buffer back.
 template <typename F>
 int with_idle_memory(int device, F&& call) {
-  for (;;) {
-    const int rc = call();
-    if (rc != DD_ERR_OOM) return rc;
-    cudaGetLastError();
-    if (!pool().drop(device)) return rc;
-  }
+  int rc = call();
+  if (rc != DD_ERR_OOM) return rc;
+  cudaGetLastError();
+  if (!pool().drop(device)) return rc;
+  rc = call();
+  if (rc == DD_ERR_OOM) cudaGetLastError();
+  return rc;
 }
 template <typename F>
 int with_idle_memory(dd_index* h, F&& call) {

@@ -161,3 +161,32 @@ def test_ground_truth_with_little_memory_left(dtype, nq):
     np.testing.assert_array_equal(ids, wi)
     np.testing.assert_array_equal(ds, wd)
     gi.close()
+
+
+def _mixed_search():
+    both = D.gen_mixture_f32(35_000, 24, 40, 3)
+    base, q = both[:5_000], both[5_000:]
+    Ls = np.resize(np.array([10, 20, 50, 100, 200], np.uint32), len(q))
+
+    def handle():
+        gi = GpuIndex(base.dtype, "l2", 5_000, 24, 24)
+        gi.upload_points(base)
+        gi.build(48, 1.2)
+        return gi
+
+    return handle, q, Ls
+
+
+def test_a_search_whose_scratch_does_not_fit_fails():
+    handle, q, Ls = _mixed_search()
+    gi = handle()
+    with free_memory(40):
+        for _ in range(2):
+            with pytest.raises(DDError, match="memory"):
+                gi.search(q, 10, Ls)
+    got = gi.search(q, 10, Ls)
+    gi.close()
+    gi = handle()
+    for a, b in zip(gi.search(q, 10, Ls), got):
+        np.testing.assert_array_equal(a, b)
+    gi.close()
