@@ -359,10 +359,11 @@ class Staging {
   uint8_t* heap_ = nullptr;
 };
 
-// (a 2-D copy refuses such a stride, stage_rows does not look at it)
-int check_query_stride(dd_index* h, uint64_t qstride) {
+// (a 2-D copy refuses such a stride, stage_rows does not look at it; 0 stands for
+// a single row's, as NumPy has it for q[None])
+int check_query_stride(dd_index* h, uint64_t qstride, uint64_t nq) {
   const uint64_t rb = (uint64_t)h->d * esize(h->dtype);
-  if (qstride >= rb) return DD_OK;
+  if (qstride >= rb || (nq == 1 && qstride == 0)) return DD_OK;
   return fail(h, DD_ERR_ARG, "query stride %llu < row bytes %llu", (unsigned long long)qstride,
               (unsigned long long)rb);
 }
@@ -1700,7 +1701,7 @@ static int search(dd_index* h, const void* queries, uint64_t nq, uint64_t qstrid
                   uint32_t* visited, uint32_t* cmps) {
   if (!h || !queries || !L_per_query || !ids || !dists) return DD_ERR_ARG;
   if (nq == 0) return DD_OK;
-  int rc = check_query_stride(h, qstride);
+  int rc = check_query_stride(h, qstride, nq);
   if (rc) return rc;
   CK(cudaSetDevice(h->device));
   const uint64_t rb = (uint64_t)h->d * esize(h->dtype), ds = h->stride;
@@ -1988,7 +1989,7 @@ int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
   if (!h || !queries || !ids || !dists) return DD_ERR_ARG;
   if (k == 0 || k > 32 || k > h->n) return fail(h, DD_ERR_UNSUPPORTED, "k must be in [1, 32]");
   if (nq == 0) return DD_OK;
-  if (const int rc = check_query_stride(h, qstride)) return rc;
+  if (const int rc = check_query_stride(h, qstride, nq)) return rc;
   CK(cudaSetDevice(h->device));
   // the lists take 1 KB a query and segment: as many queries at a time as keep the
   // workspace within 2 GB, but at least 4096 (a float base is converted once a batch)

@@ -66,3 +66,19 @@ def test_query_rows_closer_than_their_length_are_refused(nq):
             gi._ck(gi.lib.dd_groundtruth(gi.h, p(q), nq, stride, 5, p(ids), p(ds)))
     gi.search(q, 5, 20)  # the handle goes on
     gi.close()
+
+
+def test_a_single_query_without_a_stride(oracle_mod):
+    base = D.gen_skewed_u8(500, 120, 8, 5)
+    gi = GpuIndex(base.dtype, "l2", 500, 120, 16)
+    gi.upload_points(base)
+    gi.build(32, 1.2)
+    q = base[7][None]
+    assert q.strides[0] == 0
+    oi, od = oracle_mod.groundtruth(base, q, 5)
+    ids, ds = gi.groundtruth(q, 5)
+    np.testing.assert_array_equal(ids, oi)
+    np.testing.assert_array_equal(ds, od)
+    np.testing.assert_array_equal(gi.search(q, 5, 20)[0],
+                                  gi.search(base[7:8].copy(), 5, 20)[0])
+    gi.close()
