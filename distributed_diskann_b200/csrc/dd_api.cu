@@ -1615,7 +1615,6 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
   // widest class first.  Each has its own scratch; the first of a group waits for
   // the group before.
   constexpr int kLanes = 3;
-  uint64_t warps[kLanes] = {}, hwords[kLanes] = {};
   for (int c = query_class(Lmax); c >= 0; c--) {
     if (!((classes >> c) & 1u)) continue;
     if ((16u << c) < k && c < query_class(Lmax)) break;  // no valid beam width below k
@@ -1631,9 +1630,6 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
     const int wpc = r.plan.warps_per_cta;
     r.grid = (int)std::min<uint64_t>((nq + wpc - 1) / wpc,
                                      (uint64_t)r.plan.blocks_per_sm * h->sm_count);
-    const int s = (nruns - 1) % kLanes;
-    warps[s] = std::max(warps[s], (uint64_t)r.grid * wpc);
-    if (r.hglob) hwords[s] = std::max(hwords[s], (uint64_t)r.grid * wpc * r.lay.hash_words);
     // a call whose queries are all resident at once in the widest layout takes
     // one launch of it: the classes one after another add their latencies (1500
     // host queries of L = 10 to 200 on 1M x 128 uint8 2.99 -> 1.37 ms, 100 of them
@@ -1651,19 +1647,43 @@ int search_on_device(dd_index* h, const void* queries, uint64_t nq, uint64_t qst
     launch_bin_queries(L_per_query, nq, k, Lmax, h->qcls, counts, h->stream);
     h->launches++;
   }
-  const uint64_t hsum = hwords[0] + hwords[1] + hwords[2];
-  int rc = ev_slices(warps[0] + warps[1] + warps[2]);
-  if (!rc && hsum > h->qhash_words) {
+  uint64_t warps[kLanes], hwords[kLanes];  // scratch of each lane
+  auto room = [&](int lanes) -> int {
+    uint64_t wsum = 0, hsum = 0;
+    for (int s = 0; s < kLanes; s++) warps[s] = hwords[s] = 0;
+    for (int i = 0; i < nruns; i++) {
+      const ClassRun& r = runs[i];
+      const uint64_t w = (uint64_t)r.grid * r.plan.warps_per_cta;
+      warps[i % lanes] = std::max(warps[i % lanes], w);
+      if (r.hglob) hwords[i % lanes] = std::max(hwords[i % lanes], w * r.lay.hash_words);
+    }
+    for (int s = 0; s < lanes; s++) {
+      wsum += warps[s];
+      hsum += hwords[s];
+    }
+    int rc = ev_slices(wsum);
+    if (rc || hsum <= h->qhash_words) return rc;
     dfree(h->qhash);
     h->qhash = nullptr;
     h->qhash_words = 0;
     CK(dalloc(&h->qhash, hsum));
     h->qhash_words = hsum;
+    return DD_OK;
+  };
+  int lanes = std::min(kLanes, nruns);
+  int rc = with_idle_memory(h, [&] { return room(lanes); });
+  if (rc == DD_ERR_OOM && lanes > 1) {
+    // no memory for scratch side by side: one class after another
+    dfree(h->qev);
+    h->qev = nullptr;
+    h->qev_words = 0;
+    lanes = 1;
+    rc = room(lanes);
   }
   if (rc) return rc;
   for (int i = 0; i < nruns; i++) {
     const ClassRun& r = runs[i];
-    const int s = i % kLanes;
+    const int s = i % lanes;
     QueryArgs qc = qa;
     qc.Lmax = r.L;
     qc.cls_items = one ? nullptr : h->qcls + (uint64_t)r.c * nq;

@@ -190,3 +190,25 @@ def test_a_search_whose_scratch_does_not_fit_fails():
     for a, b in zip(gi.search(q, 10, Ls), got):
         np.testing.assert_array_equal(a, b)
     gi.close()
+
+
+def test_mixed_widths_with_little_memory_left():
+    """Scratch for classes that overlap does not fit; the classes run one by one."""
+    import torch
+
+    handle, q, Ls = _mixed_search()
+    gi = handle()
+    torch.cuda.empty_cache()
+    before, _ = torch.cuda.mem_get_info()
+    want = gi.search(q, 10, Ls)
+    need = (before - torch.cuda.mem_get_info()[0]) // MB
+    gi.close()
+    gi = handle()
+    gi.search(q[:5], 10, 200)  # (a first call of few queries)
+    with free_memory(need * 3 // 4):
+        got = gi.search(q, 10, Ls)
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+    for a, b in zip(gi.search(q, 10, Ls), want):
+        np.testing.assert_array_equal(a, b)
+    gi.close()
