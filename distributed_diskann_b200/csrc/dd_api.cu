@@ -71,6 +71,8 @@ struct dd_index {
   float* snorm = nullptr;
   uint64_t sstride = 0;
   bool screen_ok = false;
+  bool norms_ok = false;      // `norms` is of the present points (sharded build)
+  bool points_lent = false;   // dd_device_points: the caller may write them at any time
   bool verbose = false;
   bool hash32 = false;  // DD_HASH32=1: 32-bit hash-table ids even when n < 2^24 - 1
   int search_mode = DD_MODE_FAST;
@@ -957,7 +959,7 @@ int dd_check_errors(dd_index* h) {
 
 int dd_upload_points(dd_index* h, const void* rows, uint64_t row_stride_bytes) {
   if (!h || !rows) return DD_ERR_ARG;
-  h->screen_ok = false;  // the BF16 row copies follow the new points
+  h->screen_ok = h->norms_ok = false;  // copies and norms follow the new points
   uint64_t rb = (uint64_t)h->d * esize(h->dtype);
   if (row_stride_bytes < rb) return fail(h, DD_ERR_ARG, "row stride %llu < row bytes %llu",
                                          (unsigned long long)row_stride_bytes, (unsigned long long)rb);
@@ -970,7 +972,7 @@ int dd_upload_points(dd_index* h, const void* rows, uint64_t row_stride_bytes) {
 
 int dd_upload_points_device(dd_index* h, const void* rows, uint64_t row_stride_bytes) {
   if (!h || !rows) return DD_ERR_ARG;
-  h->screen_ok = false;  // the BF16 row copies follow the new points
+  h->screen_ok = h->norms_ok = false;  // copies and norms follow the new points
   uint64_t rb = (uint64_t)h->d * esize(h->dtype);
   if (row_stride_bytes < rb) return fail(h, DD_ERR_ARG, "row stride too small");
   CK(cudaSetDevice(h->device));
@@ -982,7 +984,7 @@ int dd_upload_points_device(dd_index* h, const void* rows, uint64_t row_stride_b
 
 int dd_upload_points_async(dd_index* h, const void* rows, uint64_t row_stride_bytes) {
   if (!h || !rows) return DD_ERR_ARG;
-  h->screen_ok = false;  // the BF16 row copies follow the new points
+  h->screen_ok = h->norms_ok = false;  // copies and norms follow the new points
   uint64_t rb = (uint64_t)h->d * esize(h->dtype);
   if (row_stride_bytes < rb) return fail(h, DD_ERR_ARG, "row stride %llu < row bytes %llu",
                                          (unsigned long long)row_stride_bytes, (unsigned long long)rb);
@@ -997,7 +999,7 @@ int dd_upload_points_async(dd_index* h, const void* rows, uint64_t row_stride_by
 // the next one is read from disk.
 int dd_load_points_file(dd_index* h, const char* path) {
   if (!h || !path) return DD_ERR_ARG;
-  h->screen_ok = false;  // the BF16 row copies follow the new points
+  h->screen_ok = h->norms_ok = false;  // copies and norms follow the new points
   std::ifstream f(path, std::ios::binary);
   if (!f) return fail(h, DD_ERR_IO, "cannot open %s", path);
   uint32_t hdr[2];
@@ -1401,6 +1403,7 @@ static int shard_begin(dd_index* h, const dd_build_params* P, uint64_t max_batch
     if (rc) return rc;
   }
   if (bp.fast && !h->norms && greedy_uses_mma(h->d, h->dtype)) CK(dalloc(&h->norms, h->n));
+  h->norms_ok = false;
   CK(cudaMemsetAsync(h->graph, 0xff, h->n * h->Rp * 4ull, h->stream));
   CK(cudaMemsetAsync(h->err, 0, 4, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -1420,6 +1423,7 @@ int dd_shard_search_prune(dd_index* h, uint64_t lo, uint64_t hi, uint32_t* rows)
   if (hi < lo || hi > h->n || hi - lo > h->shard_bmax) return fail(h, DD_ERR_ARG, "bad slice");
   if (hi == lo) return DD_OK;
   CK(cudaSetDevice(h->device));
+  h->launches = 2;  // k_search, k_prune
   BuildPlan bp = shard_plan(h);
   RoundArgs ra = shard_round_args(h, lo, hi - lo, rows);
   if (bp.fast) {
@@ -1435,7 +1439,11 @@ int dd_shard_search_prune(dd_index* h, uint64_t lo, uint64_t hi, uint32_t* rows)
   }
   if (bp.fast) {
     ix.fgroup_lg = fast_fgroup(h);
-    if (h->norms) launch_row_norms(ix, h->norms, h->stream);  // the points may have changed
+    if (h->norms && (!h->norms_ok || h->points_lent)) {  // n rows: once a build, not a round
+      launch_row_norms(ix, h->norms, h->stream);
+      h->launches++;
+      h->norms_ok = true;
+    }
     ix.norms = h->norms;
   }
   launch_search(ix, ra, bp.slay, bp.splan, grid_for(bp.splan, ra.B, h->sm_count), h->stream);
@@ -2052,6 +2060,7 @@ int dd_groundtruth(dd_index* h, const void* queries, uint64_t nq, uint64_t qstri
 void* dd_device_points(dd_index* h) {
   if (!h) return nullptr;
   h->screen_ok = false;
+  h->points_lent = true;
   return h->points;
 }
 uint64_t dd_device_row_stride(dd_index* h) { return h ? h->stride : 0; }

@@ -252,7 +252,7 @@ void* dd_device_points(dd_index* h);      /* n rows, dd_device_row_stride bytes 
 uint64_t dd_device_row_stride(dd_index* h);
 void* dd_device_graph(dd_index* h);       /* n rows of dd_device_row_len uint32 */
 uint32_t dd_device_row_len(dd_index* h);
-/* kernels launched by the last dd_build / dd_search call */
+/* kernels launched by the last dd_build / dd_search / dd_shard_search_prune call */
 uint64_t dd_last_launch_count(dd_index* h);
 
 #ifdef __cplusplus
