@@ -148,44 +148,6 @@ struct DistIntIP {
   }
 };
 
-// exact integer value of the integer forms (ground truth)
-template <int DT, int MT>
-struct DistIntRaw {
-  static __device__ __forceinline__ int eval(const void* av, const void* bv, uint32_t d) {
-    const uint4* a = (const uint4*)av;
-    const uint4* b = (const uint4*)bv;
-    uint32_t nv = (d + 15) >> 4;
-    if (MT == DD_L2) {
-      uint32_t acc = 0;
-      for (uint32_t i = 0; i < nv; i++) {
-        uint4 x = a[i], y = __ldg(b + i);
-        uint32_t t;
-        t = absdiff4<DT>(x.x, y.x); acc = __dp4a(t, t, acc);
-        t = absdiff4<DT>(x.y, y.y); acc = __dp4a(t, t, acc);
-        t = absdiff4<DT>(x.z, y.z); acc = __dp4a(t, t, acc);
-        t = absdiff4<DT>(x.w, y.w); acc = __dp4a(t, t, acc);
-      }
-      return (int)acc;
-    }
-    int acc = 0;
-    for (uint32_t i = 0; i < nv; i++) {
-      uint4 x = a[i], y = __ldg(b + i);
-      if (DT == DD_U8) {
-        acc = (int)__dp4a(x.x, y.x, (uint32_t)acc);
-        acc = (int)__dp4a(x.y, y.y, (uint32_t)acc);
-        acc = (int)__dp4a(x.z, y.z, (uint32_t)acc);
-        acc = (int)__dp4a(x.w, y.w, (uint32_t)acc);
-      } else {
-        acc = __dp4a((int)x.x, (int)y.x, acc);
-        acc = __dp4a((int)x.y, (int)y.y, acc);
-        acc = __dp4a((int)x.z, (int)y.z, acc);
-        acc = __dp4a((int)x.w, (int)y.w, acc);
-      }
-    }
-    return -acc;
-  }
-};
-
 template <> struct Dist<DD_I8, DD_L2> : DistIntL2<DD_I8> {};
 template <> struct Dist<DD_U8, DD_L2> : DistIntL2<DD_U8> {};
 template <> struct Dist<DD_I8, DD_MIPS> : DistIntIP<DD_I8> {};
