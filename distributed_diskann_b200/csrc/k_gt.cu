@@ -21,7 +21,7 @@
 //
 // Integer data: one score per pair, 2 q.p - |p|^2 (L2) or q.p (MIPS), exact in
 // 32 bits; the list keeps the k best.  Float data: rows are split x = hi + lo
-// (two BF16 values, |x - hi - lo| <= 2^-18 |x|) and the score is hi.hi + hi.lo
+// (two BF16 values, |x - hi - lo| <= 2^-17 |x|) and the score is hi.hi + hi.lo
 // + lo.hi in FP32, whose distance from the true one is at most e (gt_error);
 // the list keeps every value within 2 e of the k-th best, which holds the true
 // k best, and only those get the FP64 distance of the definition.  A query
@@ -310,16 +310,17 @@ __global__ void __launch_bounds__(256) k_gt_prep(const uint8_t* rows, uint64_t s
 }
 
 // How far the float score of any base point can lie from the exact one (of the
-// query with norm qn, base norms up to P): the three bf16 products leave out
-// lo.lo and the halves' residues (3.1 2^-18 of sum |q_i p_i| <= |q| |p|), the
-// tensor core adds at most 3 d products in FP32 (each addition 2^-23 of the
+// query with norm qn, base norms up to P).  Rounding to 8 bits leaves |lo| <=
+// 2^-8 |x| and, below the last bit of lo, a residue of at most 2^-17 |x|, so
+// lo.lo' (2^-16) and two residues (2^-17 each) are left out of the three bf16
+// products: 1.01 2^-15 of sum |q_i p_i| <= |q| |p|.  The tensor core adds at most 3 d products in FP32 (each addition 2^-23 of the
 // absolute sum, which the splitting raises by less than 2%), |p|^2 and the
 // final multiply-add round once each; 2% and an absolute term for subnormal
 // products are added.  The FP64 distances the result is ordered by are far
 // inside that margin of the real ones.
 __device__ __forceinline__ float gt_error(float qn2, float pn2, uint32_t d, bool l2) {
   const float q = sqrtf(qn2) * 1.0001f, P = sqrtf(pn2) * 1.0001f;
-  const float c = 3.1f * 0x1p-18f + 1.02f * (float)(3 * d + 64) * 0x1p-23f;
+  const float c = 1.01f * 0x1p-15f + 1.02f * (float)(3 * d + 64) * 0x1p-23f;
   const float dot = q * P;
   const float e = l2 ? 2.f * dot * c + 0x1p-22f * (2.f * dot + P * P) : dot * (c + 0x1p-22f);
   const float room = 4.f * dot + 4.f * P * P;  // no score can overflow
