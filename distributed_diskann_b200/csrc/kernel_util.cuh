@@ -3,6 +3,8 @@
 #pragma once
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
+#include <unordered_map>
 #include <vector>
 
 #include "dd_common.cuh"
@@ -65,9 +67,26 @@ __device__ __forceinline__ uint64_t warp_next_item(uint32_t* q, uint64_t& cur, u
     else { CALL4(DT, MT, 16, 4); }                                                   \
   } while (0)
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory.  The limit is
+// the process's, and a launch on another thread may need more at the same time: it
+// is only ever raised.
+inline void raise_smem_limit(const void* kernel, size_t bytes) {
+  struct Limits {
+    std::mutex mu;
+    std::unordered_map<const void*, size_t> most;
+  };
+  static Limits* limits = new Limits;  // no destructor: other threads may still launch
+  std::lock_guard<std::mutex> g(limits->mu);
+  size_t& most = limits->most[kernel];
+  const size_t want = std::max(most, bytes);
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want) ==
+      cudaSuccess)
+    most = want;
+}
+
 template <typename K>
 static void set_smem(K kernel, size_t bytes) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  raise_smem_limit((const void*)kernel, bytes);
 }
 
 template <typename K>
