@@ -29,10 +29,12 @@
 // against every point.
 //
 // Measured on B200, all kernels of a call: 10,000 x 1M x 128 uint8, k = 32: 144
-// ms (mma.sync tiles of 16 queries a warp) -> 4.4 ms; 1000 x 400k x 200 float
-// inner product: 185 ms (FP64 on the CUDA cores, one row per lane) -> 1.2 ms.
-// What bounds it now: the epilogue (two instructions a value, and the lists),
-// not the products (0.6 ms of the uint8 call at the measured GEMM rate).
+// ms (mma.sync tiles of 16 queries a warp) -> 4.34 ms (norms 0.09, sample 0.47,
+// thresholds 0.02, lists 3.68, merge 0.08); 1000 x 400k x 200 float inner product:
+// 185 ms (FP64 on the CUDA cores, one row per lane) -> 1.17 ms (halves 0.16, sample
+// 0.14, lists 0.77, merge 0.09).  What bounds it now: the epilogue (two
+// instructions a value, and the lists), not the products (0.6 ms of the uint8
+// call at the measured GEMM rate).
 #include <cfloat>
 #include <climits>
 #include <cstdio>
@@ -155,8 +157,8 @@ constexpr uint32_t kGtTileBytes = kGtTile * kGtBlockBytes;
 // The lists are in global memory (L2): appends are stores that nothing waits
 // for, and with the sample's thresholds about 50 values come to a list, so that
 // it is hardly ever compacted.  (In shared memory a list held 48: some warp
-// compacted one in most steps, and the step's TMEM buffer waited for it: 4.3 ms
-// instead of 3.7 ms for the uint8 call below.)
+// compacted one in most steps, and the step's TMEM buffer waited for it: the
+// lists of the uint8 call above took 4.3 ms instead of 3.7.)
 constexpr uint32_t kGtCap = 128;
 // |p|^2 of the rows past n, and the scores that no point lies below and no such
 // row reaches (integer rows of 1024 bytes: scores above -2^27)
@@ -179,9 +181,10 @@ struct GtShape {
 // are reduced to each group's largest, and the k-th largest of those is a
 // score that at least k points reach.  A list that starts from nothing takes
 // about k ln(points / k) values of its segment, one that starts from the
-// sample's threshold a fraction of that, and lists are dearer than products:
-// without a sample 14.7 ms (10,000 x 1M x 128 uint8) and 6.6 ms (1000 x 400k x
-// 200 float), with 1/16 of the base 6.6 / 1.1, 1/8 5.4 / 0.9, 1/4 4.6 / 1.0.
+// sample's threshold a fraction of that, and lists are dearer than products.
+// Whole host calls, 10,000 x 1M x 128 uint8 and 1000 x 400k x 200 float: without a
+// sample 26.4 and 9.04 ms, with 1/16 of the base 9.2 and 1.22, 1/8 4.85 and 1.22,
+// 1/5 4.74 and 1.24, 1/4 4.83 and 1.30.
 // A base of few tiles is sampled whole, a group a tile (99 x 67,546 x 87 uint8
 // 1.48 ms without the sample); one of fewer than k tiles is not.
 constexpr uint32_t kGtGroups = 128, kGtSampleOf = 5;

@@ -1523,13 +1523,15 @@ __device__ SearchOut warp_build_search(const SearchParams& P, const SearchSmem& 
 // multiset, and the caller runs warp_beam_search instead.
 //
 // A query is bound by the latency of its steps (15 searches share an SM at L =
-// 100, where the reference's 12 KB filter tables fill the shared memory), so
-// what counts here is the length of the chain from a row to the next one.
-// Measured on B200, k_query against warp_beam_search's: one query of 100k x 64
-// f32 at L = 100 361 -> 301 us, 10,000 at L = 50 1.39 -> 1.22 ms, 10,000 of 100k
-// x 100 int8 at L = 200 5.16 -> 4.70 ms, 50,000 inner-product queries of 400k x
-// 200 f32 at L = 50 10.9 -> 10.6 ms, 10,000 of 1M x 128 uint8 at L = 100 2.41 ->
-// 2.36 ms; at L = 10 (14 steps, mostly fetching code) 71.7 -> 73 us.
+// 100: the reference's 12 KB filter tables fill the shared memory, and 128
+// registers a thread would allow one more), so what counts here is the length of the chain from a row to the next one.
+// Measured on B200, device calls after an L2 flush, warp_beam_search -> this: one
+// query of 100k x 64 f32 at L = 100 415 -> 362 us, 10,000 at L = 50 1.34 -> 1.15
+// ms; 10,000 of 1M x 128 uint8 at L = 50 1.57 -> 1.46, at 100 2.38 -> 2.32; of 400k
+// x 200 f32 inner product at L = 50 2.75 -> 2.65. L = 10 (14 steps, mostly fetching
+// code): 10,000 of 1M x 128 uint8 550 -> 546 us, of 100k x 64 f32 519 -> 482, but
+// one integer query 79.0 -> 81.5. At L = 16 that one is 1% faster and 10,000 are 1
+// to 16%, so every width up to 256 comes here.
 // ---------------------------------------------------------------------------
 template <int DT, int MT, int FPL, int CPL>
 __device__ bool warp_query_search(const SearchParams& P, const SearchSmem& S, uint32_t self_id,
