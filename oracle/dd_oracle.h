@@ -2,7 +2,7 @@
  *
  * A plain C++ restatement of the reference algorithm (ParlayANN Vamana as
  * forked by distributed_diskann), used by tests/, __graft_entry__.smoke() and
- * bench.py's cpu_baseline leg as the checker.  The product library never
+ * bench.py's cpu_baseline leg, to compare with.  The product library never
  * links, loads or calls it.  Parity is pinned by tests/test_oracle_pin.py
  * against outputs of the reference's own sources (oracle/_ref/ref_harness)
  * committed as golden fixtures under tests/golden/.

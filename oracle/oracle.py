@@ -1,7 +1,7 @@
 """ctypes wrapper of the CPU oracle (oracle/dd_oracle.cpp) — TEST INFRASTRUCTURE.
 
 Only tests/, ``__graft_entry__.smoke()`` and bench.py's CPU-baseline leg import
-this module, and only as the checker.  The product package never does.
+this module, and only to compare with.  The product package never does.
 
 Also drives the reference's own sources built as ``oracle/_ref/ref_harness``
 (see oracle/Makefile) to pin the oracle and to time the reference CPU path.
